@@ -247,19 +247,6 @@ template <int N, int V = 0> struct Plan {
 
 constexpr int kFftThreads = 256;  // threads per CTA of every FFT kernel
 
-// Bank spread of a 16-line layout.  Lanes 0-15 and 16-31 of a warp hold one
-// element index apart (j and j + 1).  A pitch of 16 (mod 32) puts the two
-// half-warps in opposite halves of the bank space for every read and every
-// write of a later stage (element offsets 1 or odd).  A first-stage (span 1)
-// write puts the two half-warps R elements apart: for even R that is the same
-// half.  So there the upper half-warp writes its R outputs rotated by one,
-// which makes the offset R + 1 (or 1), odd again.  Every output is still
-// written once, with the same value.
-template <int NL, int PITCH, int R>
-struct RotateFirst {
-  static constexpr bool value = NL == 16 && PITCH % 32 == 16 && R % 2 == 0;
-};
-
 template <int N, int R, int NS, bool INV, int NL, int PITCH>
 CB_DEVICE void fft_stage(const float* __restrict__ sre, const float* __restrict__ sim,
                          float* __restrict__ dre, float* __restrict__ dim, const float2* __restrict__ tw) {
@@ -286,23 +273,11 @@ CB_DEVICE void fft_stage(const float* __restrict__ sre, const float* __restrict_
     }
     Dft<R, INV>::run(v);
     const int o = (j - k) * R + k;
-    if constexpr (NS == 1 && RotateFirst<NL, PITCH, R>::value) {
-      const int h = j & 1;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int rr = (r + h == R) ? 0 : r + h;
-        const float2 x = h ? v[(r + 1) % R] : v[r];
-        const int idx = (o + rr) * PITCH + p;
-        dre[idx] = x.x;
-        dim[idx] = x.y;
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int idx = (o + r * NS) * PITCH + p;
-        dre[idx] = v[r].x;
-        dim[idx] = v[r].y;
-      }
+    for (int r = 0; r < R; ++r) {
+      const int idx = (o + r * NS) * PITCH + p;
+      dre[idx] = v[r].x;
+      dim[idx] = v[r].y;
     }
   }
 }
@@ -319,127 +294,66 @@ CB_DEVICE void fft_lines(float* re, float* im, float* sre, float* sim, const flo
   __syncthreads();
 }
 
-// Column layout (lines are columns of a strided array; the thread's line p is
-// threadIdx.x % NL in every stage because kFftThreads % NL == 0): the first
-// stage can read its inputs straight from global memory and the last one
-// write its outputs straight back, the warp's lanes covering NL adjacent
-// columns at one element (coalesced).  The arithmetic is fft_stage's, so
-// results are bit-identical to staging the lines in shared memory first.
-
-// First stage (span 1: no twiddles) reading element e of the thread's line p
-// through ld(p, e) (a float2), into (dre, dim).
-template <int N, int R, bool INV, int NL, int PITCH, class Load>
-CB_DEVICE void fft_stage_in(const Load& ld, float* __restrict__ dre, float* __restrict__ dim) {
-  constexpr int J = N / R;
-  constexpr int total = NL * J;
-  static_assert(kFftThreads % NL == 0, "a thread keeps its line across stages");
-#pragma unroll 2
-  for (int u = threadIdx.x; u < total; u += kFftThreads) {
-    const int p = u % NL;
-    const int j = u / NL;
-    float2 v[R];
+// A butterfly j: elements j + R1 r through ld(e), radix-R0 transform, sums
+// k0 handed to put(k0, value).
+template <int R0, int R1, bool INV, class Load, class Put>
+CB_DEVICE void fft_a(int j, const Load& ld, const Put& put) {
+  float2 v[R0];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = ld(p, j + r * J);
-    Dft<R, INV>::run(v);
-    if constexpr (RotateFirst<NL, PITCH, R>::value) {
-      const int h = j & 1;
+  for (int r = 0; r < R0; ++r) v[r] = ld(j + R1 * r);
+  Dft<R0, INV>::run(v);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int rr = (r + h == R) ? 0 : r + h;
-        const float2 x = h ? v[(r + 1) % R] : v[r];
-        const int idx = (j * R + rr) * PITCH + p;
-        dre[idx] = x.x;
-        dim[idx] = x.y;
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int idx = (j * R + r) * PITCH + p;
-        dre[idx] = v[r].x;
-        dim[idx] = v[r].y;
-      }
-    }
-  }
+  for (int k0 = 0; k0 < R0; ++k0) put(k0, v[k0]);
 }
 
-// Last stage (span NS) from (sre, sim), handing element e of line p to
-// st(p, e, value).
-template <int N, int R, int NS, bool INV, int NL, int PITCH, class Store>
-CB_DEVICE void fft_stage_out(const float* __restrict__ sre, const float* __restrict__ sim,
-                             const float2* __restrict__ tw, const Store& st) {
-  constexpr int J = N / R;
-  constexpr int total = NL * J;
-  static_assert(kFftThreads % NL == 0, "a thread keeps its line across stages");
-#pragma unroll 2
-  for (int u = threadIdx.x; u < total; u += kFftThreads) {
-    const int p = u % NL;
-    const int j = u / NL;
-    const int k = j % NS;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int idx = (j + r * J) * PITCH + p;
-      v[r] = make_float2(sre[idx], sim[idx]);
-    }
-    if (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        float2 w = tw[r * k * (N / (NS * R))];
-        if (INV) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    Dft<R, INV>::run(v);
-    const int o = (j - k) * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) st(p, o + r * NS, v[r]);
-  }
+// Twiddle W_N^m (its conjugate for the inverse) from the table in shared memory.
+// A volatile load: the forward and the inverse half of B use the same R1
+// twiddles, and keeping them in registers in between costs occupancy.
+template <bool INV>
+CB_DEVICE float2 twiddle(const float2* tw, int m) {
+  float2 w;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
+               : "=f"(w.x), "=f"(w.y)
+               : "r"((unsigned)__cvta_generic_to_shared(tw + m)));
+  if (INV) w.y = -w.y;
+  return w;
 }
 
-// The two for a column of complex elements colp[e * es] (colp null: zeros in,
-// nothing out).
-struct ColumnLoad {
-  const float2* colp;
-  long long es;
-  CB_DEVICE float2 operator()(int, int e) const {
-    return colp ? __ldg(colp + (long long)e * es) : make_float2(0.f, 0.f);
-  }
-};
-struct ColumnStore {
-  float2* colp;
-  long long es;
-  CB_DEVICE void operator()(int, int e, float2 v) const {
-    if (colp) colp[(long long)e * es] = v;
-  }
-};
-
-// Shared-memory lines (re, im) as a stage's destination.
-template <int PITCH>
-struct SmemStore {
-  float* re;
-  float* im;
-  CB_DEVICE void operator()(int p, int e, float2 v) const {
-    re[e * PITCH + p] = v.x;
-    im[e * PITCH + p] = v.y;
-  }
-};
-
-template <int N, int R, bool INV, int NL, int PITCH>
-CB_DEVICE void fft_stage_load(const float2* __restrict__ colp, long long es, float* __restrict__ dre,
-                              float* __restrict__ dim) {
-  fft_stage_in<N, R, INV, NL, PITCH>(ColumnLoad{colp, es}, dre, dim);
+// First half of B butterfly k0: the sums through get(j), twiddled and
+// transformed: v[k1] is the spectrum at k0 + R0 k1.  (The twiddles sit here
+// and not in A so that A needs no table: its global loads start at once.)
+template <int R0, int R1, bool INV, class Get>
+CB_DEVICE void fft_b(int k0, const float2* tw, float2 (&v)[R1], const Get& get) {
+  v[0] = get(0);
+#pragma unroll
+  for (int j = 1; j < R1; ++j) v[j] = cmul(get(j), twiddle<INV>(tw, j * k0));
+  Dft<R1, INV>::run(v);
 }
 
-template <int N, int R, int NS, bool INV, int NL, int PITCH>
-CB_DEVICE void fft_stage_store(const float* __restrict__ sre, const float* __restrict__ sim,
-                               const float2* __restrict__ tw, float2* __restrict__ colp, long long es) {
-  fft_stage_out<N, R, NS, INV, NL, PITCH>(sre, sim, tw, ColumnStore{colp, es});
+// Inverse of fft_b: spectrum in v, twiddled sums to put(j, value).
+template <int R0, int R1, class Put>
+CB_DEVICE void fft_b_inverse(int k0, const float2* tw, float2 (&v)[R1], const Put& put) {
+  Dft<R1, true>::run(v);
+  put(0, v[0]);
+#pragma unroll
+  for (int j = 1; j < R1; ++j) put(j, cmul(v[j], twiddle<true>(tw, j * k0)));
 }
 
-// Stage the N-entry twiddle table into shared memory.
-template <int N>
+// Inverse of fft_a: sums through get(k0), elements j + R1 r to st(e, value).
+template <int R0, int R1, class Get, class Store>
+CB_DEVICE void fft_a_inverse(int j, const Get& get, const Store& st) {
+  float2 v[R0];
+#pragma unroll
+  for (int k0 = 0; k0 < R0; ++k0) v[k0] = get(k0);
+  Dft<R0, true>::run(v);
+#pragma unroll
+  for (int r = 0; r < R0; ++r) st(j + R1 * r, v[r]);
+}
+
+// Stage the N-entry twiddle table into shared memory (T threads).
+template <int N, int T = kFftThreads>
 CB_DEVICE void load_twiddles(float2* dst, const float2* __restrict__ src) {
-  for (int i = threadIdx.x; i < N; i += kFftThreads) dst[i] = src[i];
+  for (int i = threadIdx.x; i < N; i += T) dst[i] = src[i];
 }
 
 }  // namespace cb
