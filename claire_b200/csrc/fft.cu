@@ -68,26 +68,38 @@ bool fft_size_supported(int n) {
 
 bool fft_col_size_supported(int n) { return fft_size_supported(n) || n == 150; }
 
-// Packed lines per CTA for row kernels, and columns per CTA for column kernels.
-// With 256 threads and at least 32 lines a warp's lanes are 32 consecutive
-// lines at one element index in every radix stage, so the split re / im
-// arrays (odd line pitch) are read and written without bank conflicts; grids
-// of 192 and 256 points use 16 lines to keep two CTAs per SM.  Variant bit 1
-// selects the alternative line counts the autotuner tries (row chunks must
-// split into whole float4 per thread: P * N % 512 == 0; the 4-field pencil of
-// 256 points keeps 16 columns to fit shared memory).
-template <int N> struct RowLines {
-  static constexpr int base = N <= 32 ? 64 : (N <= 128 ? 32 : 16);
-  static constexpr int alt = N == 16 ? 32 : (N == 32 ? 32 : (N == 48 ? 64 : (N <= 128 ? 16 : 32)));
-};
+// Columns per CTA of the column kernels; variant bit 1 selects the alternative
+// count the autotuner tries.
 template <int N> struct ColLines {
   static constexpr int base = N <= 128 ? 32 : 16;
   static constexpr int alt = N <= 128 ? 16 : (N == 192 ? 32 : 16);
 };
-template <int N, int V = 0> struct RowCfg {
-  static constexpr int P = (V & 2) ? RowLines<N>::alt : RowLines<N>::base;
-  static constexpr int PITCH = P + 1;
+
+// Packed lines (row pairs) per CTA of the row kernels: a power of two P with
+// one thread per A butterfly (P * R1), 256 threads at most (128: variant bit 1).
+constexpr int row_pairs(int r1, int v) {
+  int p = 1;
+  while (2 * p * r1 <= ((v & 2) ? 128 : 256)) p *= 2;
+  return p;
+}
+
+// Row kernels (bound by global traffic: three 256^3 fields 68 us r2c and 70 us
+// c2r against a floor of 62; 150 and 165 us when rows were transposed through
+// padded shared memory on the way in and out; 128^3: 12.4 and 11.4 against 20
+// and 21): a warp's lanes are neighbouring butterflies of a few lines, so
+// the shared layout y[line, k0, j] at line * PL + k0 * PK + j is read and
+// written without bank conflicts: A (lanes over j, then lines) needs
+// PL = R1 (mod 16 float2), B (lanes over k0) an odd PK.
+template <int N, int V> struct RowCfg {
+  static constexpr int R0 = RowPlan<N, V>::R0, R1 = RowPlan<N, V>::R1;
+  static constexpr int P = row_pairs(R1, V), T = P * R1;
+  static constexpr int PK = R1 + 1;
+  static constexpr int PL = R0 * PK + ((R1 - R0 * PK) % 16 + 16) % 16;
+  static constexpr int NH = N / 2 + 1;
+  static constexpr size_t smem = (size_t)(P * PL + N) * sizeof(float2);
+  static_assert(T % 32 == 0 && (P * R0) % 32 == 0 && R1 % 2 == 0 && (R0 & (R0 - 1)) == 0, "whole warps of partners");
 };
+
 // Column kernels are bound by global traffic (each pass reads and writes its
 // spectra once) once their instructions and barriers are few.  Lanes run over
 // adjacent columns in both butterflies, so
@@ -103,209 +115,184 @@ template <int N, int V = 0> struct ColCfg {
   static_assert(T % C == 0, "a thread keeps its column");
 };
 
-constexpr int kThreads = kFftThreads;
+CB_DEVICE bool epi_reduces(int epi) { return epi == EPI_SUMSQ || epi == EPI_STORE_DOT || epi == EPI_ADD_DOT; }
 
-// Epilogue of the row kernels: value of row r, element e sits at
-// ((r & 1) ? im : re)[e * PITCH + r / 2]; store it, add it to dst, or
-// accumulate its square.  For EPI_ADD the old values of a group of 8 elements
-// are loaded before any of them is stored, so the loads overlap.
-template <int N, int P, int PITCH>
-CB_DEVICE double rows_epilogue(const float* re, const float* im, float* __restrict__ dst,
-                               const float* __restrict__ other, int row0, int nr, int epi, float al) {
-  constexpr int TOTAL = 2 * P * N;
-  constexpr int G = 8;
-  const bool add = (epi == EPI_ADD || epi == EPI_ADD_DOT);
-  const bool dot = (epi == EPI_STORE_DOT || epi == EPI_ADD_DOT);
-  double acc = 0.0;
-  for (int i0 = threadIdx.x; i0 < TOTAL; i0 += G * kThreads) {
-    float old[G], oth[G];
+// ---------------------------------------------------------------------------
+// rows (x3).  Two real rows a, b (2p and 2p + 1) are packed as z = a + i b.
+// Elements go straight between global memory and the A butterfly's registers:
+// the lanes of a line cover R1 consecutive floats, so with R1 = 8 every 32-byte
+// sector of an access is used whole.
+// ---------------------------------------------------------------------------
+template <class F>
+CB_DEVICE void rows_a(const float* __restrict__ ra, bool ok, int p, int j, float2* S) {
+  const float* rb = ra + F::R0 * F::R1;
+  fft_a<F::R0, F::R1, false>(j, [&](int e) { return ok ? make_float2(__ldg(ra + e), __ldg(rb + e)) : make_float2(0.f, 0.f); },
+                             [&](int k0, float2 v) { S[p * F::PL + k0 * F::PK + j] = v; });
+}
+
+// Inverse A butterfly and the epilogue: value e of row a / b is al times the
+// real / imaginary part; stored, added to dst, or squared and summed
+// (returned), with the product with `oth` summed for the dot epilogues.  Old
+// values of a group of elements are loaded before any of them is stored.
+template <class F>
+CB_DEVICE double rows_out(float* __restrict__ da, const float* __restrict__ oa, bool ok, int p, int j,
+                          const float2* S, int epi, float al) {
+  constexpr int R0 = F::R0, R1 = F::R1, N = R0 * R1, G = R0 < 8 ? R0 : 8;
+  float2 v[R0];
 #pragma unroll
-    for (int u = 0; u < G; ++u) {
-      const int idx = i0 + u * kThreads;
-      const int r = idx / N, e = idx - r * N;
-      const bool in = idx < TOTAL && r < nr;
-      const long long gi = (long long)(row0 + r) * N + e;
-      old[u] = (add && in) ? dst[gi] : 0.f;
-      oth[u] = (dot && in) ? other[gi] : 0.f;
+  for (int k0 = 0; k0 < R0; ++k0) v[k0] = S[p * F::PL + k0 * F::PK + j];
+  Dft<R0, true>::run(v);
+  double acc = 0.0;
+  if (!ok) return acc;
+  if (epi == EPI_STORE) {
+#pragma unroll
+    for (int r = 0; r < R0; ++r) {
+      da[j + R1 * r] = al * v[r].x;
+      da[N + j + R1 * r] = al * v[r].y;
+    }
+    return acc;
+  }
+  if (epi == EPI_SUMSQ) {
+#pragma unroll
+    for (int r = 0; r < R0; ++r) {
+      const float x = al * v[r].x, y = al * v[r].y;
+      acc += (double)x * (double)x + (double)y * (double)y;
+    }
+    return acc;
+  }
+  const bool add = (epi == EPI_ADD || epi == EPI_ADD_DOT), dot = epi != EPI_ADD;
+#pragma unroll
+  for (int r0 = 0; r0 < R0; r0 += G) {
+    float2 old[G], oth[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) {
+      const int e = j + R1 * (r0 + i);
+      old[i] = add ? make_float2(da[e], da[N + e]) : make_float2(0.f, 0.f);
+      oth[i] = dot ? make_float2(oa[e], oa[N + e]) : make_float2(0.f, 0.f);
     }
 #pragma unroll
-    for (int u = 0; u < G; ++u) {
-      const int idx = i0 + u * kThreads;
-      const int r = idx / N, e = idx - r * N;
-      if (idx >= TOTAL || r >= nr) continue;
-      const float val = al * ((r & 1) ? im : re)[e * PITCH + (r >> 1)];
-      const long long gi = (long long)(row0 + r) * N + e;
-      if (epi == EPI_SUMSQ) {
-        acc += (double)val * (double)val;
-        continue;
-      }
-      const float nv = add ? old[u] + val : val;
-      dst[gi] = nv;
-      if (dot) acc += (double)nv * (double)oth[u];
+    for (int i = 0; i < G; ++i) {
+      const int e = j + R1 * (r0 + i);
+      const float x = add ? old[i].x + al * v[r0 + i].x : al * v[r0 + i].x;
+      const float y = add ? old[i].y + al * v[r0 + i].y : al * v[r0 + i].y;
+      da[e] = x;
+      da[N + e] = y;
+      if (dot) acc += (double)x * (double)oth[i].x + (double)y * (double)oth[i].y;
     }
   }
   return acc;
 }
 
-CB_DEVICE bool epi_reduces(int epi) { return epi == EPI_SUMSQ || epi == EPI_STORE_DOT || epi == EPI_ADD_DOT; }
-
-// ---------------------------------------------------------------------------
-// load helpers
-// ---------------------------------------------------------------------------
-// Row chunk: 2P contiguous real rows of N floats -> pair-packed complex lines
-// (row 2p -> real part, row 2p+1 -> imaginary part of line p).  float4 loads.
-template <int N, int P, int PITCH>
-CB_DEVICE void load_row_chunk(float* re, float* im, const float* __restrict__ src, int nr) {
-  constexpr int Q = 2 * P * N / 4;          // float4s in the chunk
-  constexpr int K = Q / kThreads;           // per thread (exact for all plans)
-  static_assert(Q % kThreads == 0, "row chunk must split evenly");
-  float4 v[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int q = threadIdx.x + k * kThreads;
-    const int r = (4 * q) / N;
-    v[k] = (r < nr) ? __ldg(reinterpret_cast<const float4*>(src) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  // lane l writes its four elements in the order rotated by l / 8, so the 32
-  // lanes of each store hit 32 distinct banks (e * PITCH strides otherwise
-  // fold four lanes onto one bank)
-  const int rot = (threadIdx.x >> 3) & 3;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const int q = threadIdx.x + k * kThreads;
-    const int r = (4 * q) / N, e = 4 * q - r * N;
-    float* dst = ((r & 1) ? im : re) + (r >> 1);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = (i + rot) & 3;
-      const float val = c == 0 ? v[k].x : (c == 1 ? v[k].y : (c == 2 ? v[k].z : v[k].w));
-      dst[(e + c) * PITCH] = val;
-    }
-  }
+CB_DEVICE float2 shfl2(float2 v, int lane) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
 }
 
-// ---------------------------------------------------------------------------
-// rows: r2c along x3.  Two real rows a, b are packed as z = a + i b; after
-// the complex FFT Z, A[k] = (Z[k] + conj Z[N-k]) / 2, B[k] = (Z[k] - conj Z[N-k]) / 2i.
-// ---------------------------------------------------------------------------
-template <int N, int V>
-__global__ void __launch_bounds__(kThreads) k_r2c_rows(const float* __restrict__ in, long long ip,
-                                                        long long ifs, float2* __restrict__ out,
-                                                        long long op, long long ofs, int nrows,
-                                                        const float2* __restrict__ twg,
-                                                        const int* __restrict__ active) {
-  constexpr int P = RowCfg<N, V>::P, PITCH = RowCfg<N, V>::PITCH, NH = N / 2 + 1;
-  if (active && !active[blockIdx.z]) return;
-  extern __shared__ float smem[];
-  float2* tw = reinterpret_cast<float2*>(smem);
-  float* re = smem + 2 * N;
-  float* im = re + N * PITCH;
-  float* sre = im + N * PITCH;
-  float* sim = sre + N * PITCH;
-  const float* src = in + blockIdx.z * ip + blockIdx.y * ifs;
-  float2* dst = out + blockIdx.z * op + blockIdx.y * ofs;
-  const int row0 = blockIdx.x * 2 * P;
-  const int nr = min(2 * P, nrows - row0);
-  load_twiddles<N>(tw, twg);
-  load_row_chunk<N, P, PITCH>(re, im, src + (long long)row0 * N, nr);
-  __syncthreads();
-  fft_lines<N, false, P, PITCH, V>(re, im, sre, sim, tw);
-  for (int idx = threadIdx.x; idx < 2 * P * NH; idx += kThreads) {
-    const int r = idx / NH, k = idx - r * NH;
-    if (r >= nr) continue;
-    const int line = r >> 1;
-    const int km = (k == 0) ? 0 : N - k;
-    const float zr = re[k * PITCH + line], zi = im[k * PITCH + line];
-    const float mr = re[km * PITCH + line], mi = im[km * PITCH + line];
-    float2 x;
-    if (r & 1) x = make_float2(0.5f * (zi + mi), -0.5f * (zr - mr));
-    else x = make_float2(0.5f * (zr + mr), 0.5f * (zi - mi));
-    dst[(long long)(row0 + r) * NH + k] = x;
-  }
+// Lane that holds B butterfly (R0 - k0) mod R0 of this lane's line: the
+// butterflies of a line sit in R0 neighbouring lanes of one warp.
+template <int R0>
+CB_DEVICE int mirror_lane(int k0) {
+  return (int)(threadIdx.x & 31 & ~(R0 - 1)) | ((R0 - k0) & (R0 - 1));
 }
 
-// ---------------------------------------------------------------------------
-// rows: c2r along x3 with epilogue.  Z[k] = A[k] + i B[k], Z[N-k] =
-// conj(A[k]) + i conj(B[k]); the imaginary parts of the DC and Nyquist bins
-// are ignored (the c2r convention of FFTW / pocketfft).
-// ---------------------------------------------------------------------------
+// r2c: after the complex FFT Z of a row pair, A[k] = (Z[k] + conj Z[N-k]) / 2,
+// B[k] = (Z[k] - conj Z[N-k]) / 2i.  Z[N-k] is in the mirror lane's registers,
+// element R1 - 1 - k1 (butterfly 0 mirrors itself, element R1 - k1).
 template <int N, int V>
-__global__ void __launch_bounds__(kThreads) k_c2r_rows(const float2* __restrict__ in, long long ip,
-                                                        long long ifs, float* __restrict__ out,
-                                                        long long op, long long ofs, int nrows,
-                                                        const float2* __restrict__ twg, int epi,
-                                                        const float* __restrict__ alpha,
-                                                        double* __restrict__ partials, int nparts,
-                                                        const float* __restrict__ other,
-                                                        const int* __restrict__ active) {
-  constexpr int P = RowCfg<N, V>::P, PITCH = RowCfg<N, V>::PITCH, NH = N / 2 + 1;
+__global__ void __launch_bounds__(RowCfg<N, V>::T, 1024 / RowCfg<N, V>::T)
+    k_r2c_rows(const float* __restrict__ in, long long ip, long long ifs, float2* __restrict__ out, long long op,
+               long long ofs, int nrows, const float2* __restrict__ twg, const int* __restrict__ active) {
+  using F = RowCfg<N, V>;
+  constexpr int R0 = F::R0, R1 = F::R1, NH = F::NH;
   if (active && !active[blockIdx.z]) return;
-  extern __shared__ float smem[];
-  float2* tw = reinterpret_cast<float2*>(smem);
-  float* re = smem + 2 * N;
-  float* im = re + N * PITCH;
-  float* sre = im + N * PITCH;
-  float* sim = sre + N * PITCH;
-  // staging of the 2P half-spectrum rows: it is dead before the transform
-  // starts, so it shares the transform's scratch (sre / sim) when that is large
-  // enough (row_smem sizes the block for the larger of the two)
-  float* str = sre;
-  float* sti = str + 2 * P * NH;
-  const float2* src = in + blockIdx.z * ip + blockIdx.y * ifs;
-  float* dst = out ? out + blockIdx.z * op + blockIdx.y * ofs : nullptr;
-  const float* oth = other ? other + blockIdx.z * op + blockIdx.y * ofs : nullptr;
-  const int row0 = blockIdx.x * 2 * P;
-  const int nr = min(2 * P, nrows - row0);
-  load_twiddles<N>(tw, twg);
+  extern __shared__ __align__(16) float2 sm2[];
+  float2* tw = sm2 + F::P * F::PL;
+  const int row0 = blockIdx.x * 2 * F::P;
+  load_twiddles<N, F::T>(tw, twg);
   {
-    // two-phase load of the 2P x NH complex chunk (contiguous)
-    constexpr int TOT = 2 * P * NH;
-    constexpr int K = (TOT + kThreads - 1) / kThreads;
-    const float2* s0 = src + (long long)row0 * NH;
-    float2 v[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int idx = threadIdx.x + k * kThreads;
-      v[k] = (idx < TOT && idx / NH < nr) ? __ldg(s0 + idx) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const int idx = threadIdx.x + k * kThreads;
-      if (idx >= TOT) continue;
-      const int kk = idx % NH;
-      float2 w = v[k];
-      if (kk == 0 || kk == N / 2) w.y = 0.f;
-      str[idx] = w.x;
-      sti[idx] = w.y;
-    }
+    const int p = threadIdx.x / R1, j = threadIdx.x % R1, row = row0 + 2 * p;
+    const float* src = in + blockIdx.z * ip + blockIdx.y * ifs + (long long)row * N;
+    rows_a<F>(src, row < nrows, p, j, sm2);
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < P * N; idx += kThreads) {
-    const int line = idx / N, e = idx - line * N;
-    const int a = 2 * line, b = 2 * line + 1;
-    float zr, zi;
-    if (e <= N / 2) {
-      const float ar = str[a * NH + e], ai = sti[a * NH + e];
-      const float br = str[b * NH + e], bi = sti[b * NH + e];
-      zr = ar - bi;
-      zi = ai + br;
-    } else {
-      const int k = N - e;
-      const float ar = str[a * NH + k], ai = -sti[a * NH + k];
-      const float br = str[b * NH + k], bi = -sti[b * NH + k];
-      zr = ar - bi;
-      zi = ai + br;
+  float2* dst = out + blockIdx.z * op + blockIdx.y * ofs;
+  for (int u = threadIdx.x; u < F::P * R0; u += F::T) {
+    const int p = u / R0, k0 = u % R0, row = row0 + 2 * p;
+    float2 v[R1];
+    fft_b<R0, R1, false>(k0, tw, v, [&](int j) { return sm2[p * F::PL + k0 * F::PK + j]; });
+    const int lane = mirror_lane<R0>(k0);
+    const bool ok = row < nrows;
+    float2* da = dst + (long long)row * NH + k0;
+#pragma unroll
+    for (int k1 = 0; k1 < R1 / 2; ++k1) {
+      float2 m = shfl2(v[R1 - 1 - k1], lane);
+      if (k0 == 0) m = v[k1 == 0 ? 0 : R1 - k1];
+      const float2 z = v[k1];
+      if (ok) {
+        da[R0 * k1] = make_float2(0.5f * (z.x + m.x), 0.5f * (z.y - m.y));
+        da[NH + R0 * k1] = make_float2(0.5f * (z.y + m.y), -0.5f * (z.x - m.x));
+      }
     }
-    re[e * PITCH + line] = zr;
-    im[e * PITCH + line] = zi;
+    if (ok && k0 == 0) {  // Nyquist
+      da[N / 2] = make_float2(v[R1 / 2].x, 0.f);
+      da[NH + N / 2] = make_float2(v[R1 / 2].y, 0.f);
+    }
+  }
+}
+
+// c2r with epilogue: Z[k] = A[k] + i B[k], Z[N-k] = conj(A[k]) + i conj(B[k])
+// handed to the mirror lane; the imaginary parts of the DC and Nyquist bins
+// are ignored (the c2r convention of FFTW / pocketfft).
+template <int N, int V>
+__global__ void __launch_bounds__(RowCfg<N, V>::T, 1024 / RowCfg<N, V>::T)
+    k_c2r_rows(const float2* __restrict__ in, long long ip, long long ifs, float* __restrict__ out, long long op,
+               long long ofs, int nrows, const float2* __restrict__ twg, int epi, const float* __restrict__ alpha,
+               double* __restrict__ partials, int nparts, const float* __restrict__ other,
+               const int* __restrict__ active) {
+  using F = RowCfg<N, V>;
+  constexpr int R0 = F::R0, R1 = F::R1, NH = F::NH, H = R1 / 2;
+  if (active && !active[blockIdx.z]) return;
+  extern __shared__ __align__(16) float2 sm2[];
+  float2* tw = sm2 + F::P * F::PL;
+  const int row0 = blockIdx.x * 2 * F::P;
+  load_twiddles<N, F::T>(tw, twg);
+  __syncthreads();
+  const float2* src = in + blockIdx.z * ip + blockIdx.y * ifs;
+  for (int u = threadIdx.x; u < F::P * R0; u += F::T) {
+    const int p = u / R0, k0 = u % R0, row = row0 + 2 * p;
+    const bool ok = row < nrows;
+    const float2* sa = src + (long long)row * NH + k0;
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 v[R1], hi[H];
+#pragma unroll
+    for (int k1 = 0; k1 < H; ++k1) {
+      v[k1] = ok ? __ldg(sa + R0 * k1) : zero;
+      hi[k1] = ok ? __ldg(sa + NH + R0 * k1) : zero;
+    }
+    float2 nyq = zero;
+    if (k0 == 0) {
+      if (ok) nyq = make_float2(__ldg(sa + N / 2).x, __ldg(sa + NH + N / 2).x);
+      v[0].y = hi[0].y = 0.f;
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < H; ++k1) {
+      const float2 a = v[k1], b = hi[k1];
+      v[k1] = make_float2(a.x - b.y, a.y + b.x);
+      hi[k1] = make_float2(a.x + b.y, b.x - a.y);
+    }
+    const int lane = mirror_lane<R0>(k0);
+#pragma unroll
+    for (int k1 = 0; k1 < H; ++k1) {
+      const float2 m = shfl2(hi[k1], lane);
+      v[R1 - 1 - k1] = k0 ? m : (k1 + 1 < H ? hi[k1 + 1 < H ? k1 + 1 : 0] : nyq);
+    }
+    fft_b_inverse<R0, R1>(k0, tw, v, [&](int j, float2 x) { sm2[p * F::PL + k0 * F::PK + j] = x; });
   }
   __syncthreads();
-  fft_lines<N, true, P, PITCH, V>(re, im, sre, sim, tw);
-  const float al = alpha ? alpha[blockIdx.z] : 1.f;
-  const double acc = rows_epilogue<N, P, PITCH>(re, im, dst, oth, row0, nr, epi, al);
-  if (epi_reduces(epi)) {
+  const int p = threadIdx.x / R1, j = threadIdx.x % R1, row = row0 + 2 * p;
+  const long long off = blockIdx.z * op + blockIdx.y * ofs + (long long)row * N;
+  const double acc = rows_out<F>(out + off, other + off, row < nrows, p, j, sm2, epi, alpha ? alpha[blockIdx.z] : 1.f);
+  if (epi_reduces(epi))
     block_reduce_store(acc, partials + (long long)blockIdx.z * nparts, blockIdx.x + gridDim.x * blockIdx.y);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -641,45 +628,42 @@ __global__ void __launch_bounds__(ColCfg<N, V>::T, 512 / ColCfg<N, V>::T) k_penc
 // and imaginary parts of the result are the derivatives of a and b.
 // AXIS 2: rows (x3, contiguous).  AXIS 0/1: columns along x1 / x2.
 // ---------------------------------------------------------------------------
-template <int N, int NL, int PITCH>
-CB_DEVICE void mul_ik(float* re, float* im, float hscale) {
-  for (int idx = threadIdx.x; idx < NL * N; idx += kThreads) {
-    const int e = idx / NL, p = idx - e * NL;
-    const float k = (float)wavenumber(e, N) * hscale;
-    const int a = e * PITCH + p;
-    const float xr = re[a], xi = im[a];
-    re[a] = -k * xi;
-    im[a] = k * xr;
+// i k / N on the outputs k0 + R0 k1 of a B butterfly
+template <int N, int R0, int R1>
+CB_DEVICE void mul_ik(int k0, float2 (&v)[R1]) {
+#pragma unroll
+  for (int k1 = 0; k1 < R1; ++k1) {
+    const float k = (float)wavenumber(k0 + R0 * k1, N) * (1.f / (float)N);
+    v[k1] = make_float2(-k * v[k1].y, k * v[k1].x);
   }
 }
 
 template <int N, int V>
-__global__ void __launch_bounds__(kThreads) k_deriv_rows(const float* __restrict__ in, long long ip,
-                                                          long long ifs, float* __restrict__ out,
-                                                          long long op, long long ofs, int nrows,
-                                                          const float2* __restrict__ twg, int epi,
-                                                          double* __restrict__ partials, int nparts,
-                                                          const int* __restrict__ active) {
-  constexpr int P = RowCfg<N, V>::P, PITCH = RowCfg<N, V>::PITCH;
+__global__ void __launch_bounds__(RowCfg<N, V>::T, 1024 / RowCfg<N, V>::T)
+    k_deriv_rows(const float* __restrict__ in, long long ip, long long ifs, float* __restrict__ out, long long op,
+                 long long ofs, int nrows, const float2* __restrict__ twg, int epi, double* __restrict__ partials,
+                 int nparts, const int* __restrict__ active) {
+  using F = RowCfg<N, V>;
+  constexpr int R0 = F::R0, R1 = F::R1;
   if (active && !active[blockIdx.z]) return;
-  extern __shared__ float smem[];
-  float2* tw = reinterpret_cast<float2*>(smem);
-  float* re = smem + 2 * N;
-  float* im = re + N * PITCH;
-  float* sre = im + N * PITCH;
-  float* sim = sre + N * PITCH;
-  const float* src = in + blockIdx.z * ip + blockIdx.y * ifs;
-  float* dst = out ? out + blockIdx.z * op + blockIdx.y * ofs : nullptr;
-  const int row0 = blockIdx.x * 2 * P;
-  const int nr = min(2 * P, nrows - row0);
-  load_twiddles<N>(tw, twg);
-  load_row_chunk<N, P, PITCH>(re, im, src + (long long)row0 * N, nr);
+  extern __shared__ __align__(16) float2 sm2[];
+  float2* tw = sm2 + F::P * F::PL;
+  const int row0 = blockIdx.x * 2 * F::P;
+  const int p = threadIdx.x / R1, j = threadIdx.x % R1, row = row0 + 2 * p;
+  load_twiddles<N, F::T>(tw, twg);
+  rows_a<F>(in + blockIdx.z * ip + blockIdx.y * ifs + (long long)row * N, row < nrows, p, j, sm2);
   __syncthreads();
-  fft_lines<N, false, P, PITCH, V>(re, im, sre, sim, tw);
-  mul_ik<N, P, PITCH>(re, im, 1.f / (float)N);
+  for (int u = threadIdx.x; u < F::P * R0; u += F::T) {
+    const int k0 = u % R0;
+    float2* S = sm2 + (u / R0) * F::PL + k0 * F::PK;
+    float2 v[R1];
+    fft_b<R0, R1, false>(k0, tw, v, [&](int i) { return S[i]; });
+    mul_ik<N, R0, R1>(k0, v);
+    fft_b_inverse<R0, R1>(k0, tw, v, [&](int i, float2 x) { S[i] = x; });
+  }
   __syncthreads();
-  fft_lines<N, true, P, PITCH, V>(re, im, sre, sim, tw);
-  const double acc = rows_epilogue<N, P, PITCH>(re, im, dst, nullptr, row0, nr, epi, 1.f);
+  const double acc = rows_out<F>(out + blockIdx.z * op + blockIdx.y * ofs + (long long)row * N, nullptr,
+                                 row < nrows && (out || epi == EPI_SUMSQ), p, j, sm2, epi, 1.f);
   if (epi == EPI_SUMSQ)
     block_reduce_store(acc, partials + (long long)blockIdx.z * nparts, blockIdx.x + gridDim.x * blockIdx.y);
 }
@@ -721,11 +705,7 @@ __global__ void __launch_bounds__(ColCfg<N, V>::T, 1024 / ColCfg<N, V>::T) k_der
   for (int k0 = u0; k0 < R0; k0 += F::T / C) {
     float2 v[R1];
     fft_b<R0, R1, false>(k0, tw, v, [&](int j) { return sm2[(k0 * R1 + j) * C + c]; });
-#pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) {
-      const float k = (float)wavenumber(k0 + R0 * k1, N) * (1.f / (float)N);
-      v[k1] = make_float2(-k * v[k1].y, k * v[k1].x);
-    }
+    mul_ik<N, R0, R1>(k0, v);
     fft_b_inverse<R0, R1>(k0, tw, v, [&](int j, float2 x) { sm2[(k0 * R1 + j) * C + c] = x; });
   }
   __syncthreads();
@@ -759,12 +739,6 @@ __global__ void __launch_bounds__(ColCfg<N, V>::T, 1024 / ColCfg<N, V>::T) k_der
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-template <int N, int V> static size_t row_smem(bool c2r) {
-  const size_t scratch = 2 * N * RowCfg<N, V>::PITCH;           // sre + sim
-  const size_t staging = 2 * 2 * RowCfg<N, V>::P * (N / 2 + 1);  // c2r half-spectrum rows (shares scratch)
-  const size_t tail = (c2r && staging > scratch) ? staging : scratch;
-  return (2 * N + 2 * N * RowCfg<N, V>::PITCH + tail) * sizeof(float);
-}
 // nbuf exchange buffers, the twiddles and (symbol) the pencil's symbol table
 template <int N, int V> static size_t col_smem(int nbuf, bool symbol = false) {
   return (size_t)(nbuf * ColCfg<N, V>::B + N) * sizeof(float2) + (symbol ? ColCfg<N, V>::B * sizeof(float) : 0);
@@ -907,11 +881,11 @@ static int r2c_rows_impl(const float* in, long long ip, long long ifs, float2* o
                          cudaStream_t s) {
   const float2* tw = twiddles(N);
   if (!tw) return (int)cudaErrorMemoryAllocation;
-  size_t sm = row_smem<N, V>(false);
+  size_t sm = RowCfg<N, V>::smem;
   int e = set_smem(k_r2c_rows<N, V>, sm);
   if (e) return e;
   dim3 grid((nrows + 2 * RowCfg<N, V>::P - 1) / (2 * RowCfg<N, V>::P), nf, nprob);
-  k_r2c_rows<N, V><<<grid, kThreads, sm, s>>>(in, ip, ifs, out, op, ofs, nrows, tw, active);
+  k_r2c_rows<N, V><<<grid, RowCfg<N, V>::T, sm, s>>>(in, ip, ifs, out, op, ofs, nrows, tw, active);
   return (int)cudaGetLastError();
 }
 
@@ -921,11 +895,11 @@ static int c2r_rows_impl(const float2* in, long long ip, long long ifs, float* o
                          double* partials, int nparts, const float* other, const int* active, cudaStream_t s) {
   const float2* tw = twiddles(N);
   if (!tw) return (int)cudaErrorMemoryAllocation;
-  size_t sm = row_smem<N, V>(true);
+  size_t sm = RowCfg<N, V>::smem;
   int e = set_smem(k_c2r_rows<N, V>, sm);
   if (e) return e;
   dim3 grid((nrows + 2 * RowCfg<N, V>::P - 1) / (2 * RowCfg<N, V>::P), nf, nprob);
-  k_c2r_rows<N, V><<<grid, kThreads, sm, s>>>(in, ip, ifs, out, op, ofs, nrows, tw, epi, alpha, partials,
+  k_c2r_rows<N, V><<<grid, RowCfg<N, V>::T, sm, s>>>(in, ip, ifs, out, op, ofs, nrows, tw, epi, alpha, partials,
                                             nparts, other, active);
   return (int)cudaGetLastError();
 }
@@ -1006,20 +980,23 @@ int launch_pencil(float2* spec, long long sp, int nprob, const Dims& d, int op,
 // Lines per CTA of the size's current variant (min_over_variants: the
 // smallest over its candidates, which sizes reduction buffers for any variant).
 static int row_lines(int n, bool min_over_variants = false) {
-  int base = 0, alt = 0;
-  switch (n) {
-    case 16: base = RowLines<16>::base; alt = RowLines<16>::alt; break;
-    case 32: base = RowLines<32>::base; alt = RowLines<32>::alt; break;
-    case 48: base = RowLines<48>::base; alt = RowLines<48>::alt; break;
-    case 64: base = RowLines<64>::base; alt = RowLines<64>::alt; break;
-    case 96: base = RowLines<96>::base; alt = RowLines<96>::alt; break;
-    case 128: base = RowLines<128>::base; alt = RowLines<128>::alt; break;
-    case 192: base = RowLines<192>::base; alt = RowLines<192>::alt; break;
-    case 256: base = RowLines<256>::base; alt = RowLines<256>::alt; break;
-    default: return 0;
-  }
-  if (min_over_variants) return base < alt ? base : alt;
-  return (fft_variant(n) & 2) ? alt : base;
+  auto pairs = [](int k, int v) {
+    switch (k) {
+      case 16: return row_pairs((v & 1) ? RowPlan<16, 1>::R1 : RowPlan<16, 0>::R1, v);
+      case 32: return row_pairs((v & 1) ? RowPlan<32, 1>::R1 : RowPlan<32, 0>::R1, v);
+      case 48: return row_pairs((v & 1) ? RowPlan<48, 1>::R1 : RowPlan<48, 0>::R1, v);
+      case 64: return row_pairs((v & 1) ? RowPlan<64, 1>::R1 : RowPlan<64, 0>::R1, v);
+      case 96: return row_pairs((v & 1) ? RowPlan<96, 1>::R1 : RowPlan<96, 0>::R1, v);
+      case 128: return row_pairs((v & 1) ? RowPlan<128, 1>::R1 : RowPlan<128, 0>::R1, v);
+      case 192: return row_pairs((v & 1) ? RowPlan<192, 1>::R1 : RowPlan<192, 0>::R1, v);
+      case 256: return row_pairs((v & 1) ? RowPlan<256, 1>::R1 : RowPlan<256, 0>::R1, v);
+      default: return 0;
+    }
+  };
+  if (!min_over_variants) return pairs(n, fft_variant(n));
+  int m = pairs(n, 0);
+  for (int v = 1; v < 4; ++v) m = pairs(n, v) < m ? pairs(n, v) : m;
+  return m;
 }
 
 static int col_lines(int n, bool min_over_variants = false) {
@@ -1069,12 +1046,12 @@ static int deriv_rows_impl(const float* in, long long ip, long long ifs, float* 
                            const int* active, cudaStream_t s) {
   const float2* tw = twiddles(N);
   if (!tw) return (int)cudaErrorMemoryAllocation;
-  size_t sm = row_smem<N, V>(false);
+  size_t sm = RowCfg<N, V>::smem;
   int e = set_smem(k_deriv_rows<N, V>, sm);
   if (e) return e;
   const int nrows = d.n1 * d.n2;
   dim3 grid((nrows + 2 * RowCfg<N, V>::P - 1) / (2 * RowCfg<N, V>::P), nf, nprob);
-  k_deriv_rows<N, V><<<grid, kThreads, sm, s>>>(in, ip, ifs, out, op_, ofs, nrows, tw, epi, partials, nparts, active);
+  k_deriv_rows<N, V><<<grid, RowCfg<N, V>::T, sm, s>>>(in, ip, ifs, out, op_, ofs, nrows, tw, epi, partials, nparts, active);
   return (int)cudaGetLastError();
 }
 
@@ -1144,25 +1121,25 @@ static int spectral3_explicit_impl(const float* in, float* out, float2* spec, co
   const long long n = d.n(), nc = d.nc();
   const int n3h = N / 2 + 1;
   const int nrows = d.n1 * d.n2;
-  int e = set_smem(k_r2c_rows<N, V>, row_smem<N, V>(false));
+  int e = set_smem(k_r2c_rows<N, V>, RowCfg<N, V>::smem);
   if (!e) e = set_smem(k_cols<N, false, V>, col_smem<N, V>(1));
   if (!e) e = set_smem(k_cols<N, true, V>, col_smem<N, V>(1));
   if (!e) e = set_smem(k_pencil1<N, V, true>, col_smem<N, V>(1, true));
-  if (!e) e = set_smem(k_c2r_rows<N, V>, row_smem<N, V>(true));
+  if (!e) e = set_smem(k_c2r_rows<N, V>, RowCfg<N, V>::smem);
   if (e) return e;
   const dim3 rows((nrows + 2 * RowCfg<N, V>::P - 1) / (2 * RowCfg<N, V>::P), 3, 1);
   const int ncx2 = d.n1 * n3h;
   const dim3 cols((ncx2 + ColCfg<N, V>::C - 1) / ColCfg<N, V>::C, 3, 1);
   const int ncx1 = d.n2 * n3h;
   const dim3 pen((ncx1 + ColCfg<N, V>::C - 1) / ColCfg<N, V>::C, 1, 1);
-  k_r2c_rows<N, V><<<rows, kThreads, row_smem<N, V>(false), s>>>(in, 0, n, spec, 0, nc, nrows, tw, nullptr);
+  k_r2c_rows<N, V><<<rows, RowCfg<N, V>::T, RowCfg<N, V>::smem, s>>>(in, 0, n, spec, 0, nc, nrows, tw, nullptr);
   constexpr int T = ColCfg<N, V>::T;
   const size_t sm = col_smem<N, V>(1);
   k_cols<N, false, V><<<cols, T, sm, s>>>(spec, 0, nc, ncx2, n3h, (long long)d.n2 * n3h, n3h, tw, nullptr);
   k_pencil1<N, V, true><<<pen, T, col_smem<N, V>(1, true), s>>>(
       spec, 0, nc, 3, d, op, 1.f / (float)((double)d.n1 * d.n2 * d.n3), params, tw, nullptr);
   k_cols<N, true, V><<<cols, T, sm, s>>>(spec, 0, nc, ncx2, n3h, (long long)d.n2 * n3h, n3h, tw, nullptr);
-  k_c2r_rows<N, V><<<rows, kThreads, row_smem<N, V>(true), s>>>(spec, 0, nc, out, 0, n, nrows, tw, EPI_STORE, nullptr,
+  k_c2r_rows<N, V><<<rows, RowCfg<N, V>::T, RowCfg<N, V>::smem, s>>>(spec, 0, nc, out, 0, n, nrows, tw, EPI_STORE, nullptr,
                                                            nullptr, 0, nullptr, nullptr);
   return (int)cudaGetLastError();
 }

@@ -1,19 +1,16 @@
-// In-shared-memory batched complex FFT engine (mixed radix, Stockham).
+// Batched complex FFT engine: two radix stages in registers, one exchange
+// through shared memory.
 //
-// A CTA transforms `nlines` complex lines of length N that live in shared
-// memory as split real/imaginary arrays: element e of line p sits at
-// re[e*PITCH + p], im[e*PITCH + p] (line index fastest; PITCH odd for 32 or
-// more lines, so that consecutive lines hit distinct banks, and 16 for 16
-// lines, see RotateFirst).  Line count and pitch are
-// compile-time so every loop has a known trip count.  Every plan has exactly two radix
-// stages (N = R0*R1, R0, R1 in {4, 8, 10, 12, 15, 16}), each an in-register DFT
-// followed by one shared-memory exchange, so the result lands back in the
-// source buffer after one ping-pong through the scratch buffer.
-//
-// Stockham stage with radix R and span Ns (product of earlier radices):
-//   for j in [0, N/R): k = j mod Ns
-//     v[r] = x[j + r*N/R] * W_N^(r*k*N/(Ns*R));  v = DFT_R(v)
-//     y[(j - k)*R + k + r*Ns] = v[r]
+// A line of N = R0 * R1 elements is transformed by R1 "A" butterflies of radix
+// R0 and R0 "B" butterflies of radix R1.  With n = j + R1 r and k = k0 + R0 k1,
+//   X[k] = sum_j W_R1^(j k1) W_N^(j k0) sum_r x[j + R1 r] W_R0^(r k0):
+// A butterfly j reads the elements j + R1 r straight from global memory and
+// leaves its R0 sums y[k0, j] in shared memory; B butterfly k0 reads y[k0, .]
+// back, twiddles them and holds the R1 outputs k0 + R0 k1.  The inverse
+// transform runs the same two butterflies in the opposite order (B, then A), so
+// a spectral multiply sits in registers between B and its inverse: nothing is
+// reordered in between, and forward transform, symbol and inverse transform
+// take two exchanges and no other pass through shared memory.
 // Twiddles W_N^m = exp(-2*pi*i*m/N) come from a table computed on the host
 // in double precision and staged in shared memory.
 #pragma once
@@ -245,54 +242,20 @@ template <int N, int V = 0> struct Plan {
   static_assert(R0 * R1 == N, "plan must factor N");
 };
 
-constexpr int kFftThreads = 256;  // threads per CTA of every FFT kernel
-
-template <int N, int R, int NS, bool INV, int NL, int PITCH>
-CB_DEVICE void fft_stage(const float* __restrict__ sre, const float* __restrict__ sim,
-                         float* __restrict__ dre, float* __restrict__ dim, const float2* __restrict__ tw) {
-  constexpr int J = N / R;
-  constexpr int total = NL * J;
-#pragma unroll 2
-  for (int u = threadIdx.x; u < total; u += kFftThreads) {
-    const int p = u % NL;
-    const int j = u / NL;
-    const int k = j % NS;
-    float2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int idx = (j + r * J) * PITCH + p;
-      v[r] = make_float2(sre[idx], sim[idx]);
-    }
-    if (NS > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        float2 w = tw[r * k * (N / (NS * R))];
-        if (INV) w.y = -w.y;
-        v[r] = cmul(v[r], w);
-      }
-    }
-    Dft<R, INV>::run(v);
-    const int o = (j - k) * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int idx = (o + r * NS) * PITCH + p;
-      dre[idx] = v[r].x;
-      dim[idx] = v[r].y;
-    }
-  }
-}
-
-// Transform nlines lines held in (re, im); (sre, sim) is scratch of the same
-// size.  The result is back in (re, im).  Caller synchronises before; this
-// function synchronises after each stage.
-template <int N, bool INV, int NL, int PITCH, int V = 0>
-CB_DEVICE void fft_lines(float* re, float* im, float* sre, float* sim, const float2* tw) {
-  using P = Plan<N, V>;
-  fft_stage<N, P::R0, 1, INV, NL, PITCH>(re, im, sre, sim, tw);
-  __syncthreads();
-  fft_stage<N, P::R1, P::R0, INV, NL, PITCH>(sre, sim, re, im, tw);
-  __syncthreads();
-}
+// Row kernels exchange mirrored outputs between the lanes of a line, so there R0
+// is a power of two (the butterflies of a line do not straddle a warp) and R1 even.
+template <int N, int V> struct RowPlan {
+  static constexpr bool alt = (V & 1) != 0;
+  static constexpr int R0 = N == 16    ? 4
+                            : N == 32  ? (alt ? 4 : 8)
+                            : N == 48  ? (alt ? 8 : 4)
+                            : N == 64  ? (alt ? 16 : 8)
+                            : N == 96  ? (alt ? 16 : 8)
+                            : N == 128 ? (alt ? 8 : 16)
+                                       : 16;
+  static constexpr int R1 = N / R0;
+  static_assert(R0 * R1 == N, "plan must factor N");
+};
 
 // A butterfly j: elements j + R1 r through ld(e), radix-R0 transform, sums
 // k0 handed to put(k0, value).
@@ -351,7 +314,7 @@ CB_DEVICE void fft_a_inverse(int j, const Get& get, const Store& st) {
 }
 
 // Stage the N-entry twiddle table into shared memory (T threads).
-template <int N, int T = kFftThreads>
+template <int N, int T>
 CB_DEVICE void load_twiddles(float2* dst, const float2* __restrict__ src) {
   for (int i = threadIdx.x; i < N; i += T) dst[i] = src[i];
 }
