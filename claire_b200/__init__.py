@@ -300,15 +300,15 @@ def kernel_launches() -> int:
 
 
 def stage_timeouts() -> int:
-    """Tile gathers on the current device whose shared-memory box copy ran out
-    of its bounded wait (claire_b200_stage_timeouts)."""
+    """Bounded device waits that ran out on the current device
+    (claire_b200_stage_timeouts)."""
     c = ctypes.c_longlong(0)
     _check(lib.claire_b200_stage_timeouts(ctypes.byref(c)), "stage_timeouts")
     return int(c.value)
 
 
 def stage_wait_selftest(wait_ns: int = 1_000_000) -> None:
-    """Make one bounded box-copy wait run out (claire_b200_stage_wait_selftest)."""
+    """Make one bounded device wait run out (claire_b200_stage_wait_selftest)."""
     _check(lib.claire_b200_stage_wait_selftest(int(wait_ns), _stream()), "stage_wait_selftest")
 
 

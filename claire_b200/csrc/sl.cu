@@ -36,57 +36,44 @@ static int allow_smem(K kernel) {
 struct VelocitySource {
   const float* v;
   float c0, c1, c2;  // -sign*ht*N_k/(2 pi)
-  CB_DEVICE void load(float (&dd)[kTilePts][3], const TileThread& tt, const Dims& d) const {
+  CB_DEVICE void at(float (&dd)[3], unsigned i, const Dims& d) const {
     const float* v2 = v + d.n();
-    const float* v3 = v2 + d.n();
-#pragma unroll
-    for (int a = 0; a < kTilePts; ++a) {
-      const bool ok = tt.valid_idx(a);
-      const unsigned i = tt.idx(a);
-      dd[a][0] = ok ? c0 * __ldg(v + i) : 0.f;
-      dd[a][1] = ok ? c1 * __ldg(v2 + i) : 0.f;
-      dd[a][2] = ok ? c2 * __ldg(v3 + i) : 0.f;
-    }
+    dd[0] = c0 * __ldg(v + i);
+    dd[1] = c1 * __ldg(v2 + i);
+    dd[2] = c2 * __ldg(v2 + d.n() + i);
   }
 };
+
+// Epilogues of the gathers: operator()(index, value, aux) with aux =
+// epi.aux[index] loaded by the gather before it needs it (aux may be null).
 
 // Component k of X = x - sign*(ht/2)*(v + v(X~)) as a displacement:
-// disp_k = h_k (v_k + v_k(X~)), h_k = -sign*(ht/2)*N_k/(2 pi).
+// disp_k = h_k (v_k + v_k(X~)), h_k = -sign*(ht/2)*N_k/(2 pi) (aux = v_k).
 struct TrajectoryEpi {
-  const float* vk;
   float* dk;
   float h;
-  CB_DEVICE void operator()(const TileThread& tt, int a, float vx) const {
-    if (tt.valid_idx(a)) dk[tt.idx(a)] = h * (__ldg(vk + tt.idx(a)) + vx);
-  }
+  const float* aux;
+  CB_DEVICE void operator()(unsigned i, float vx, float vk) const { dk[i] = h * (vk + vx); }
 };
 
-// Epilogues of the table-driven gathers: operator()(tt, a, value, aux_a) with
-// aux_a = aux[point] prefetched by the gather (aux may be null).
 struct StoreEpi {
   float* dst;
   const float* aux = nullptr;
-  CB_DEVICE void operator()(const TileThread& tt, int a, float val, float) const {
-    if (tt.valid_idx(a)) dst[tt.idx(a)] = val;
-  }
+  CB_DEVICE void operator()(unsigned i, float val, float) const { dst[i] = val; }
 };
 
 // bf16 image output (round to nearest even)
 struct Store16Epi {
   bf16* dst;
   const float* aux = nullptr;
-  CB_DEVICE void operator()(const TileThread& tt, int a, float val, float) const {
-    if (tt.valid_idx(a)) dst[tt.idx(a)] = __float2bfloat16_rn(val);
-  }
+  CB_DEVICE void operator()(unsigned i, float val, float) const { dst[i] = __float2bfloat16_rn(val); }
 };
 
 // out = c * val (aux = c)
 struct ScaleEpi {
   float* out;
   const float* aux;
-  CB_DEVICE void operator()(const TileThread& tt, int a, float val, float c) const {
-    if (tt.valid_idx(a)) out[tt.idx(a)] = c * val;
-  }
+  CB_DEVICE void operator()(unsigned i, float val, float c) const { out[i] = c * val; }
 };
 
 // out = sign * (val + src) (aux = src)
@@ -94,9 +81,7 @@ struct AddEpi {
   float* out;
   float sign;
   const float* aux;
-  CB_DEVICE void operator()(const TileThread& tt, int a, float val, float src) const {
-    if (tt.valid_idx(a)) out[tt.idx(a)] = sign * (val + src);
-  }
+  CB_DEVICE void operator()(unsigned i, float val, float src) const { out[i] = sign * (val + src); }
 };
 
 // out = 1 + ht/2 (s dx + s dv + ht dx dv), dx = divv(X) (the gathered value),
@@ -105,8 +90,8 @@ struct AdjCoefEpi {
   float* out;
   float ht, sgn;
   const float* aux;
-  CB_DEVICE void operator()(const TileThread& tt, int a, float dx, float dv) const {
-    if (tt.valid_idx(a)) out[tt.idx(a)] = 1.f + 0.5f * ht * (sgn * (dx + dv) + ht * dx * dv);
+  CB_DEVICE void operator()(unsigned i, float dx, float dv) const {
+    out[i] = 1.f + 0.5f * ht * (sgn * (dx + dv) + ht * dx * dv);
   }
 };
 
@@ -155,87 +140,112 @@ __global__ void __launch_bounds__(256) k_field_stats(const float* __restrict__ f
 
 // ---- gather kernels (grid: tiles x problems x fields) -------------------------
 
+// The fields of a launch are split over grid.z in runs of nfz per CTA (the last
+// one shorter).
 __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
-    k_trajectory(const float* __restrict__ v, long long vp, float* __restrict__ disp, long long dp, Dims d,
-                 float ht, float sign, const int* __restrict__ active) {
-  const int p = blockIdx.y, k = blockIdx.z;
+    k_trajectory(const float* __restrict__ v, long long vp, float* __restrict__ disp, long long dp, int nfz, Dims d,
+                 TileGrid tg, float ht, float sign, const int* __restrict__ active) {
+  const int p = blockIdx.y, k0 = blockIdx.z * nfz;
   if (active && !active[p]) return;
   extern __shared__ __align__(16) float sbuf[];
   const float* v1 = v + p * vp;
   const float c0 = (float)(d.n1 / kTwoPi), c1 = (float)(d.n2 / kTwoPi), c2 = (float)(d.n3 / kTwoPi);
-  VelocitySource src{v1, -sign * ht * c0, -sign * ht * c1, -sign * ht * c2};
-  const float ck = k == 0 ? c0 : (k == 1 ? c1 : c2);
-  const float* vk = v1 + k * d.n();
-  TrajectoryEpi epi{vk, disp + p * dp + k * d.n(), -sign * 0.5f * ht * ck};
-  tile_gather(sbuf, src, vk, d, epi);
+  const VelocitySource src{v1, -sign * ht * c0, -sign * ht * c1, -sign * ht * c2};
+  const long long n = d.n();
+  tile_gather(sbuf, src, nullptr, v1 + k0 * n, n, min(nfz, 3 - k0), d, tg, [&](int i) {
+    const int k = k0 + i;
+    const float ck = k == 0 ? c0 : (k == 1 ? c1 : c2);
+    return TrajectoryEpi{disp + p * dp + k * n, -sign * 0.5f * ht * ck, v1 + k * n};
+  });
 }
 
-// field z of f (ff apart) -> field z of out (of apart)
+// fields of f (ff apart) -> fields of out (of apart); tab may be null
 __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
     k_interp(const float* __restrict__ f, long long fp, long long ff, const float* __restrict__ disp, long long dp,
-             const int4* __restrict__ tab, long long tp, float* __restrict__ out, long long op, long long of, Dims d,
-             const int* __restrict__ active) {
+             const int4* __restrict__ tab, long long tp, float* __restrict__ out, long long op, long long of, int nf,
+             int nfz, Dims d, TileGrid tg, const int* __restrict__ active) {
+  const int p = blockIdx.y, k0 = blockIdx.z * nfz;
+  if (active && !active[p]) return;
+  extern __shared__ __align__(16) float sbuf[];
+  float* o = out + p * op + k0 * of;
+  tile_gather(sbuf, DispSource{disp + p * dp}, tab ? tab + p * tp : nullptr, f + p * fp + k0 * ff, ff,
+                     min(nfz, nf - k0), d, tg, [&](int i) { return StoreEpi{o + i * of, nullptr}; });
+}
+
+// one bf16 field without a box table
+__global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
+    k_interp16_direct(const bf16* __restrict__ f, const float* __restrict__ disp, bf16* __restrict__ out, Dims d,
+                      TileGrid tg) {
+  extern __shared__ __align__(16) float sbuf[];
+  tile_gather(sbuf, DispSource{disp}, nullptr, f, 0, 1, d, tg, [&](int) { return Store16Epi{out, nullptr}; });
+}
+
+// one field with a box table (one state time step)
+__global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
+    k_interp1(const float* __restrict__ f, long long fp, const float* __restrict__ disp, long long dp,
+              const int4* __restrict__ tab, long long tp, float* __restrict__ out, long long op, Dims d, TileGrid tg,
+              const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
   extern __shared__ __align__(16) float sbuf[];
-  StoreEpi epi{out + p * op + (long long)blockIdx.z * of, nullptr};
-  tile_gather_tab(sbuf, disp + p * dp, tab + p * tp, f + p * fp + (long long)blockIdx.z * ff, d, epi);
+  StoreEpi epi{out + p * op, nullptr};
+  tile_step(sbuf, DispSource{disp + p * dp}, tab + p * tp, f + p * fp, d, tg, epi);
 }
 
 // bf16 image field of problem p -> bf16 out (one state time step)
 __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
     k_interp16(const bf16* __restrict__ f, long long fp, const float* __restrict__ disp, long long dp,
-               const int4* __restrict__ tab, long long tp, bf16* __restrict__ out, long long op, Dims d,
+               const int4* __restrict__ tab, long long tp, bf16* __restrict__ out, long long op, Dims d, TileGrid tg,
                const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
   extern __shared__ __align__(16) float sbuf[];
   Store16Epi epi{out + p * op, nullptr};
-  tile_gather_tab(sbuf, disp + p * dp, tab + p * tp, f + p * fp, d, epi);
+  tile_step(sbuf, DispSource{disp + p * dp}, tab + p * tp, f + p * fp, d, tg, epi);
 }
 
 __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
     k_gather_scale(const float* __restrict__ f, long long fp, const float* __restrict__ disp, long long dp,
                    const int4* __restrict__ tab, long long tp, const float* __restrict__ c, long long cp,
-                   float* __restrict__ out, long long op, Dims d, const int* __restrict__ active) {
+                   float* __restrict__ out, long long op, Dims d, TileGrid tg, const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
   extern __shared__ __align__(16) float sbuf[];
   ScaleEpi epi{out + p * op, c + p * cp};
-  tile_gather_tab(sbuf, disp + p * dp, tab + p * tp, f + p * fp, d, epi);
+  tile_step(sbuf, DispSource{disp + p * dp}, tab + p * tp, f + p * fp, d, tg, epi);
 }
 
 __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
     k_gather_add(const float* __restrict__ f, long long fp, const float* __restrict__ disp, long long dp,
                  const int4* __restrict__ tab, long long tp, const float* __restrict__ s, long long sp,
-                 float* __restrict__ out, long long op, float sign, Dims d, const int* __restrict__ active) {
+                 float* __restrict__ out, long long op, float sign, Dims d, TileGrid tg, const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
   extern __shared__ __align__(16) float sbuf[];
   AddEpi epi{out + p * op, sign, s + p * sp};
-  tile_gather_tab(sbuf, disp + p * dp, tab + p * tp, f + p * fp, d, epi);
+  tile_step(sbuf, DispSource{disp + p * dp}, tab + p * tp, f + p * fp, d, tg, epi);
 }
 
 __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
     k_adjoint_coef(const float* __restrict__ divv, long long vp, const float* __restrict__ disp, long long dp,
                    const int4* __restrict__ tab, long long tp, float* __restrict__ out, long long op, float ht,
-                   float sgn, Dims d, const int* __restrict__ active) {
+                   float sgn, Dims d, TileGrid tg, const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
   extern __shared__ __align__(16) float sbuf[];
   AdjCoefEpi epi{out + p * op, ht, sgn, divv + p * vp};
-  tile_gather_tab(sbuf, disp + p * dp, tab + p * tp, divv + p * vp, d, epi);
+  tile_step(sbuf, DispSource{disp + p * dp}, tab + p * tp, divv + p * vp, d, tg, epi);
 }
 
 // Box table of a displacement field (sl_tile.cuh box_from_table layout).
 __global__ void __launch_bounds__(kTileThreads)
-    k_tile_table(const float* __restrict__ disp, long long dp, int4* __restrict__ tab, long long tp, Dims d,
+    k_tile_table(const float* __restrict__ disp, long long dp, int4* __restrict__ tab, long long tp, Dims d, TileGrid tg,
                  const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
-  const TileThread tt = tile_thread(d);
+  const TileThread tt = tile_thread(d, tg);
   float dd[kTilePts][3];
-  DispSource{disp + p * dp}.load(dd, tt, d);
+  load_points(DispSource{disp + p * dp}, dd, tt, d);
   int lo[3], hi[3];
   tile_bounds(dd, tt, lo, hi);
   if (threadIdx.x == 0) {
@@ -354,11 +364,23 @@ __global__ void k_incstate_source(const float* __restrict__ gx, long long gxp, c
 
 // ---- launchers ---------------------------------------------------------------
 
+// Fields per CTA of a launch over nf fields: all of them share a CTA's set-up
+// once that leaves a full wave of CTAs (4 per SM); smaller launches run one
+// field per CTA.
+static int fields_per_cta(const Dims& d, int nprob, int nf) {
+  const long long tiles = (long long)tile_count(d) * nprob;
+  int nfz = 1;
+  while (nfz < nf && tiles * ((nf + nfz) / (nfz + 1)) >= 4 * 148) ++nfz;
+  return nfz;
+}
+
 int launch_trajectory(const float* v, long long vp, float* disp, long long dp, int nprob,
                       const Dims& d, float ht, float sign, const int* active, cudaStream_t s) {
   int e = allow_smem(k_trajectory);
   if (e) return e;
-  k_trajectory<<<tile_grid(d, nprob, 3), kTileThreads, kGatherSmemBytes, s>>>(v, vp, disp, dp, d, ht, sign, active);
+  const int nfz = fields_per_cta(d, nprob, 3);
+  k_trajectory<<<tile_grid(d, nprob, (3 + nfz - 1) / nfz), kTileThreads, kGatherSmemBytes, s>>>(
+      v, vp, disp, dp, nfz, d, TileGrid(d), ht, sign, active);
   return (int)cudaGetLastError();
 }
 
@@ -366,27 +388,47 @@ long long tile_table_int4s(const Dims& d) { return 2LL * tile_count(d); }
 
 int launch_tile_table(const float* disp, long long dp, int4* tab, long long tp, int nprob, const Dims& d,
                       const int* active, cudaStream_t s) {
-  k_tile_table<<<tile_grid(d, nprob, 1), kTileThreads, 0, s>>>(disp, dp, tab, tp, d, active);
+  k_tile_table<<<tile_grid(d, nprob, 1), kTileThreads, 0, s>>>(disp, dp, tab, tp, d, TileGrid(d), active);
   return (int)cudaGetLastError();
 }
 
 int launch_interp(const float* f, long long fp, long long ff, const float* disp, long long dp, const int4* tab,
                   long long tp, float* out, long long op, long long of, int nf, int nprob, const Dims& d,
                   const int* active, cudaStream_t s) {
+  if (nf == 1 && tab) {
+    int e = allow_smem(k_interp1);
+    if (e) return e;
+    k_interp1<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(f, fp, disp, dp, tab, tp, out, op, d,
+                                                                             TileGrid(d), active);
+    return (int)cudaGetLastError();
+  }
   int e = allow_smem(k_interp);
   if (e) return e;
-  k_interp<<<tile_grid(d, nprob, nf), kTileThreads, kGatherSmemBytes, s>>>(f, fp, ff, disp, dp, tab, tp, out, op,
-                                                                           of, d, active);
+  const int nfz = fields_per_cta(d, nprob, nf);
+  k_interp<<<tile_grid(d, nprob, (nf + nfz - 1) / nfz), kTileThreads, kGatherSmemBytes, s>>>(
+      f, fp, ff, disp, dp, tab, tp, out, op, of, nf, nfz, d, TileGrid(d), active);
   return (int)cudaGetLastError();
 }
+
+// Whether one gather at a new displacement should build its table first: the
+// table's own pass costs less than the reduction inside each gather CTA once the
+// tiles fill the GPU (256^3: 37 + 179 us against 217; 128^3: 6 + 27 against 32);
+// below that it is one more launch (64^3: 2.4 + 7.5 against 8.1).
+bool interp_wants_table(const Dims& d) { return tile_count(d) >= 4 * 148; }
 
 int launch_interp16(const bf16* f, long long fp, const float* disp, long long dp, const int4* tab, long long tp,
                     bf16* out, long long op, int nprob, const Dims& d, const int* active, cudaStream_t s) {
   // staged boxes load 4-element chunks as 8-byte words (only when N3 % 4 == 0)
   if (!(d.n3 & 3) && ((reinterpret_cast<uintptr_t>(f) & 7) || (fp & 3))) return (int)cudaErrorInvalidValue;
+  if (!tab) {
+    int e = allow_smem(k_interp16_direct);
+    if (e) return e;
+    k_interp16_direct<<<tile_grid(d, 1, 1), kTileThreads, kGatherSmemBytes, s>>>(f, disp, out, d, TileGrid(d));
+    return (int)cudaGetLastError();
+  }
   int e = allow_smem(k_interp16);
   if (e) return e;
-  k_interp16<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(f, fp, disp, dp, tab, tp, out, op, d,
+  k_interp16<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(f, fp, disp, dp, tab, tp, out, op, d, TileGrid(d),
                                                                             active);
   return (int)cudaGetLastError();
 }
@@ -397,7 +439,7 @@ int launch_gather_scale(const float* f, long long fp, const float* disp, long lo
   int e = allow_smem(k_gather_scale);
   if (e) return e;
   k_gather_scale<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(f, fp, disp, dp, tab, tp, c, cp,
-                                                                                out, op, d, active);
+                                                                                out, op, d, TileGrid(d), active);
   return (int)cudaGetLastError();
 }
 
@@ -407,7 +449,7 @@ int launch_gather_add(const float* f, long long fp, const float* disp, long long
   int e = allow_smem(k_gather_add);
   if (e) return e;
   k_gather_add<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(f, fp, disp, dp, tab, tp, src, sp,
-                                                                              out, op, sign, d, active);
+                                                                              out, op, sign, d, TileGrid(d), active);
   return (int)cudaGetLastError();
 }
 
@@ -417,7 +459,7 @@ int launch_adjoint_coef(const float* divv, long long vp, const float* disp, long
   int e = allow_smem(k_adjoint_coef);
   if (e) return e;
   k_adjoint_coef<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(divv, vp, disp, dp, tab, tp, out,
-                                                                                op, ht, sgn, d, active);
+                                                                                op, ht, sgn, d, TileGrid(d), active);
   return (int)cudaGetLastError();
 }
 
@@ -457,8 +499,7 @@ int launch_field_stats(const float* f, long long fp, long long n, int nprob, dou
   return (int)cudaGetLastError();
 }
 
-// Health of the box copies' bounded waits: tile gathers on this device whose
-// box copy did not complete within the wait limit (each skipped its tile).
+// Bounded waits on this device that ran out.
 int stage_timeouts(unsigned long long* count, cudaStream_t s) {
   unsigned v = 0;
   if (cudaMemcpyFromSymbolAsync(&v, g_stage_timeouts, sizeof(unsigned), 0, cudaMemcpyDeviceToHost, s) !=
@@ -480,7 +521,7 @@ __global__ void __launch_bounds__(kTileThreads) k_stage_wait_selftest(unsigned l
     mbar_arrive_expect(bar, 16u);
   }
   __syncthreads();
-  if (threadIdx.x == 0) stage_box_wait(bar, wait_ns);  // nothing delivers the 16 bytes
+  if (threadIdx.x == 0) bounded_wait(bar, wait_ns);  // nothing delivers the 16 bytes
 }
 
 int launch_stage_wait_selftest(unsigned long long wait_ns, cudaStream_t s) {

@@ -89,23 +89,26 @@ int launch_trajectory(const float* v, long long vp, float* disp, long long dp, i
 
 // Box table of displacement field disp[p] for the tile gathers below:
 // 2 int4 per 8x8x16 tile (tile_table_int4s(d) int4 per problem, tp apart).
-// Box copies of the tile gathers that ran out of their bounded wait (count on
-// the current device; read on stream s after its work), and a self-test that
-// makes one wait run out.
+// Bounded waits that ran out (count on the current device; read on stream s
+// after its work), and a self-test that makes one run out.
 int stage_timeouts(unsigned long long* count, cudaStream_t s = nullptr);
 int launch_stage_wait_selftest(unsigned long long wait_ns, cudaStream_t s);
 int launch_tile_table(const float* disp, long long dp, int4* tab, long long tp, int nprob, const Dims& d,
                       const int* active, cudaStream_t s);
 long long tile_table_int4s(const Dims& d);
 
+// Whether a single gather at a displacement should build its table first.
+bool interp_wants_table(const Dims& d);
+
 // out[p][f] <- f[p][f](i + disp[p](i)), f = 0..nf-1; fields ff apart; tab =
-// disp's box table.
+// disp's box table (null: every CTA reduces its box itself).
 int launch_interp(const float* f, long long fp, long long ff, const float* disp, long long dp, const int4* tab,
                   long long tp, float* out, long long op, long long of, int nf, int nprob, const Dims& d,
                   const int* active, cudaStream_t s);
 
 // Same for one bf16 image field per problem (state levels stored in bf16):
-// taps widened to FP32, sums in FP32, the result rounded to bf16.
+// taps widened to FP32, sums in FP32, the result rounded to bf16.  Without a
+// table: one problem.
 int launch_interp16(const bf16* f, long long fp, const float* disp, long long dp, const int4* tab, long long tp,
                     bf16* out, long long op, int nprob, const Dims& d, const int* active, cudaStream_t s);
 

@@ -1,31 +1,40 @@
 // Shared-memory tiled tricubic gathers.
 //
 // One CTA of 256 threads owns a tile of 8 (x1) x 8 (x2) x 16 (x3) output
-// points.  Warp w covers x2 row w of the tile; lanes 0-15 and 16-31 cover the
-// 16 x3 points of two adjacent x1 planes, and each thread holds 4 points
-// (x1 = 2a + h, a < 4, h = lane / 16).
+// points.  A warp covers 2 x2 rows of 16 x3 points, and each thread holds the 4
+// points of consecutive x1 planes in its row and column, as two pairs.
 //
-// The CTA reads its points' displacements, reduces the bounding box of every
-// stencil tap over the tile (min / max of i + floor(d), widened by the
-// stencil's -1 .. +2) and, when the box fits, copies it into shared memory
-// with bulk asynchronous copies (the TMA engine's untiled form), one per x3
-// row of the box (two where the row crosses the periodic x3 seam; the x1 / x2
-// wrap is applied per row), which complete on an mbarrier that every thread
-// waits on (bounded).  The 64 taps
-// per point are then served from shared memory; tiles whose box is too large
-// (large, rough displacements) gather from global memory instead.
+// The CTA takes the bounding box of every stencil tap over the tile (min / max of
+// i + floor(d), widened by the stencil's -1 .. +2) and, when it fits, copies it
+// into shared memory with 16-byte asynchronous copies (the periodic wrap is
+// applied per row and per chunk).  The 64 taps per point are then served from
+// shared memory; tiles whose box is too large (large, rough displacements)
+// gather from global memory instead.
 //
-// Shared-memory layout of a box: x3 rows of pitch P floats (32 or 64, a
-// multiple of 32, so lanes whose taps fall in different x2 rows still hit
-// distinct banks), x1 planes of stride Q = ext2 * P + 16 (16 mod 32: the two
-// half-warps, one plane apart, use opposite halves of the bank space).  Every
-// shared-memory index is inside the box by construction: each point's taps lie
-// in [i + floor(d) - 1, i + floor(d) + 2] and the box spans the min / max of
-// exactly those values over the tile's points; points outside the grid
-// (partial tiles) read the box origin and are never stored.
+// What bounds a gather is the shared-memory data path (64 words a point, and
+// bank conflicts on top where floors change inside a warp) and, close behind,
+// instruction issue.  The two points of a pair nearly always have the same
+// floor(d) (all but 3-10% of them on the benchmark's velocities): their stencils
+// then share 3 of 5 planes, and one pass over 5 planes of 16 words serves both
+// (40 words a point).  A pair whose floors differ gathers its first point in
+// that pass and lists the second; after a barrier the CTA gathers the listed
+// points one per thread.
+//
+// Shared-memory layout of a box: x3 rows of pitch P = 48 floats (16 mod 32: the 2
+// rows of a warp use opposite halves of the bank space), x1 planes of stride
+// Q = ext2 * P.  Every shared-memory index is inside the box by construction:
+// each point's taps lie in [i + floor(d) - 1, i + floor(d) + 2] and the box spans
+// the min / max of exactly those values over the tile's points; points outside
+// the grid (partial tiles) repeat the last point inside and are never stored.
 //
 // The kernels are not persistent: several CTAs per SM (one tile each) overlap
 // one another's copies with their gathers.
+//
+// Measured in situ, 8 problems of 128^3, all launches of a solve's first two
+// Gauss-Newton iterations: adjoint steps 161 us (173 with a stencil per point,
+// 32-bit loads of 64 words a point and a bulk copy per box row), incremental
+// steps 153 (162), state steps 181 (205), the 24 cached gradient fields 4.08 ms
+// (4.61), characteristics 0.61 ms (0.72).
 #pragma once
 
 #include <climits>
@@ -39,9 +48,13 @@ constexpr int kT1 = 8, kT2 = 8, kT3 = 16;
 constexpr int kTileThreads = 256;
 constexpr int kTilePts = 4;  // points per thread
 
-// Shared-memory budget of a CTA (one box): 4 CTAs of 256 threads per SM.
-constexpr int kGatherBudget = 8192;  // floats
-constexpr int kGatherSmemBytes = kGatherBudget * 4;
+// Shared memory of a CTA: one box and the list of single points (at most every
+// second one).  4 CTAs of 256 threads per SM; the boxes stop here because what
+// four CTAs leave of the 256 KB is the L1 cache of the displacement and operand
+// loads (11648 floats and a 9 KB list: time steps 7% slower).
+constexpr int kGatherBudget = 9856;  // floats
+constexpr int kMaxListed = kTileThreads * kTilePts / 2;
+constexpr int kGatherSmemBytes = kGatherBudget * 4 + kMaxListed * 2;
 constexpr int kGatherMinBlocks = 4;
 
 __host__ __device__ inline unsigned tile_count(const Dims& d) {
@@ -65,93 +78,124 @@ CB_DEVICE int wrap_near(int x, int n) {
   return x;
 }
 
-// This thread's points in the CTA's tile: (t1 + 2a, i2, i3), a < 4.  Point
-// indices are 32-bit (grids up to 1024^3 points).
-struct TileThread {
-  int t1, i2, i3;
-  unsigned vmask;  // bit a: point a lies inside the grid
-  unsigned idx0, step2;
-  CB_DEVICE bool valid_idx(int a) const { return (vmask >> a) & 1u; }
-  CB_DEVICE bool valid(int a, const Dims&) const { return valid_idx(a); }
-  CB_DEVICE int x1(int a) const { return t1 + 2 * a; }
-  CB_DEVICE unsigned idx(int a) const { return idx0 + a * step2; }
+// Tiles along x2 and x3 and the reciprocals that split a tile index without a
+// division: umulhi(t, floor(2^32 / nb) + 1) exceeds t / nb by at most one.
+struct TileGrid {
+  unsigned nb2, nb3, m2, m3;
+  __host__ __device__ explicit TileGrid(const Dims& d)
+      : nb2((d.n2 + kT2 - 1) / kT2), nb3((d.n3 + kT3 - 1) / kT3),
+        m2(nb2 == 1 ? 0u : (unsigned)((1ull << 32) / nb2) + 1u), m3(nb3 == 1 ? 0u : (unsigned)((1ull << 32) / nb3) + 1u) {}
 };
 
-CB_DEVICE TileThread tile_thread(const Dims& d) {
-  const int nb3 = (d.n3 + kT3 - 1) / kT3, nb2 = (d.n2 + kT2 - 1) / kT2;
-  const int t = blockIdx.x;
-  const int r = small_div(t, nb3), c3 = t - r * nb3;
-  const int c1 = small_div(r, nb2), c2 = r - c1 * nb2;
-  const int lane = threadIdx.x & 31;
+CB_DEVICE unsigned tile_div(unsigned t, unsigned nb, unsigned m) {
+  if (nb == 1) return t;
+  const unsigned q = __umulhi(t, m);
+  return q * nb > t ? q - 1 : q;
+}
+
+// x1 plane of a thread's point a, from its first.
+CB_DEVICE constexpr int plane_of(int a) { return a; }
+
+// This thread's points in the CTA's tile: 4 consecutive x1 planes of one row
+// and column.  Coordinates are clamped to the grid: a point beyond it repeats
+// the last one inside (same tile, so the same box), which makes every load and
+// every stencil valid without a predicate; only its store is left out.  Point
+// indices are 32-bit (grids up to 1024^3 points).
+struct TileThread {
+  int x1_, x2, x3;  // first plane, row, column (clamped)
+  int amax;         // planes past the first that are inside the grid
+  unsigned vmask;   // bit a: point a lies inside the grid
+  unsigned idx0, plane;
+  CB_DEVICE bool valid(int a) const { return (vmask >> a) & 1u; }
+  CB_DEVICE int step(int a) const { return min(plane_of(a), amax); }
+  CB_DEVICE int x1(int a) const { return x1_ + step(a); }
+  CB_DEVICE unsigned idx(int a) const { return idx0 + (unsigned)step(a) * plane; }
+};
+
+// Position of thread t's points in its tile (first x1 plane, x2 row, x3
+// column): a warp covers 4 planes x 2 rows x 16 columns.
+CB_DEVICE void tile_local(int t, int& l1, int& l2, int& l3) {
+  l1 = 4 * (t >> 7);
+  l2 = (t >> 4) & 7;
+  l3 = t & 15;
+}
+
+// Origin of the CTA's tile.
+CB_DEVICE void tile_origin(const TileGrid& tg, int& t1, int& t2, int& t3) {
+  const unsigned t = blockIdx.x, r = tile_div(t, tg.nb3, tg.m3), c1 = tile_div(r, tg.nb2, tg.m2);
+  t1 = (int)(c1 * kT1);
+  t2 = (int)((r - c1 * tg.nb2) * kT2);
+  t3 = (int)((t - r * tg.nb3) * kT3);
+}
+
+CB_DEVICE TileThread tile_thread(const Dims& d, const TileGrid& tg) {
+  int t1, t2, t3, l1, l2, l3;
+  tile_origin(tg, t1, t2, t3);
+  tile_local(threadIdx.x, l1, l2, l3);
+  const int p1 = t1 + l1, p2 = t2 + l2, p3 = t3 + l3;
   TileThread tt;
-  tt.t1 = c1 * kT1 + (lane >> 4);
-  tt.i2 = c2 * kT2 + (threadIdx.x >> 5);
-  tt.i3 = c3 * kT3 + (lane & 15);
-  const bool row_ok = (tt.i2 < d.n2) && (tt.i3 < d.n3);
-  tt.vmask = 0;
-#pragma unroll
-  for (int a = 0; a < kTilePts; ++a) tt.vmask |= (row_ok && tt.t1 + 2 * a < d.n1) ? (1u << a) : 0u;
-  const unsigned plane = (unsigned)d.n2 * (unsigned)d.n3;
-  tt.step2 = 2 * plane;
-  tt.idx0 = (unsigned)tt.t1 * plane + (unsigned)tt.i2 * (unsigned)d.n3 + (unsigned)tt.i3;
+  const bool row_ok = (p2 < d.n2) && (p3 < d.n3);
+  const int left = d.n1 - p1;  // planes inside the grid from p1 on
+  tt.vmask = row_ok && left > 0 ? (left >= kTilePts ? 15u : (1u << left) - 1u) : 0u;
+  tt.x1_ = min(p1, d.n1 - 1);
+  tt.x2 = min(p2, d.n2 - 1);
+  tt.x3 = min(p3, d.n3 - 1);
+  tt.amax = max(left - 1, 0);
+  tt.plane = (unsigned)d.n2 * (unsigned)d.n3;
+  tt.idx0 = (unsigned)tt.x1_ * tt.plane + (unsigned)tt.x2 * (unsigned)d.n3 + (unsigned)tt.x3;
   return tt;
 }
+
+constexpr int kPitch = 48;  // x3 row pitch of a staged box (floats, 16 mod 32 banks)
 
 struct TileBox {
   int lo[3];
   int e1, e2, e3;  // extents (e3 in whole 16-byte chunks)
-  int P, Q;        // x3 row pitch, x1 plane stride (floats)
-  int vol;         // e1 * Q, rounded up to a multiple of 32
-  bool within;     // copyable (one wrap per axis, whole chunks)
+  int Q;           // x1 plane stride (floats)
+  bool fits;       // copyable (one wrap per axis, whole chunks) and within budget
 };
 
-// Box of the stencil bases b in [lo, hi] per axis (taps b .. b+3).
+// Box of the stencil bases b = i + floor(d) - 1 in [lo, hi] per axis (taps b .. b+3).
 CB_DEVICE TileBox box_from_bounds(const int (&lo)[3], const int (&hi)[3], const Dims& d) {
+  const int nk[3] = {d.n1, d.n2, d.n3};
   TileBox bx;
   int ext[3];
-  bool within = true;
-  const int nk[3] = {d.n1, d.n2, d.n3};
+  bool fits = true;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    bx.lo[k] = lo[k];
-    const long long e = (long long)hi[k] - (long long)lo[k] + 4;
-    ext[k] = (e > 0 && e <= 4096) ? (int)e : 4096;
+    const long long l = lo[k], e = (long long)hi[k] - l + 4;
     // one wrap per coordinate in the copy, origin within one period
-    within = within && e > 0 && e <= nk[k] && lo[k] >= -nk[k] && lo[k] < nk[k];
+    fits = fits && e > 0 && e <= nk[k] && l >= -nk[k] && l < nk[k];
+    bx.lo[k] = fits ? (int)l : 0;
+    ext[k] = fits ? (int)e : 4;
   }
   // x3: start on a multiple of 4 floats and cover whole 4-float chunks so the
   // box is copied in 16-byte pieces (N3 % 4 == 0: no chunk straddles the seam)
   const int lo3a = bx.lo[2] & ~3;
   bx.e3 = ((bx.lo[2] + ext[2] - lo3a) + 3) & ~3;
   bx.lo[2] = lo3a;
-  within = within && bx.e3 <= d.n3 && bx.e3 <= 64 && (d.n3 & 3) == 0;
   bx.e1 = ext[0];
   bx.e2 = ext[1];
-  bx.P = bx.e3 <= 32 ? 32 : 64;
-  bx.Q = bx.e2 * bx.P + 16;
-  const long long vol = ((long long)bx.e1 * bx.Q + 31) & ~31LL;
-  bx.vol = vol < (1 << 24) ? (int)vol : (1 << 24);
-  bx.within = within;
+  bx.Q = bx.e2 * kPitch;
+  bx.fits = fits && bx.e3 <= d.n3 && bx.e3 <= kPitch && (d.n3 & 3) == 0 &&
+            (long long)bx.e1 * bx.Q <= kGatherBudget;
   return bx;
 }
 
-// Block-wide min / max of the stencil bases of the tile's valid points.
+// Block-wide min / max of the stencil bases of the tile's points.
 // Contains __syncthreads: call once, from uniform control flow.
 CB_DEVICE void tile_bounds(const float (&dd)[kTilePts][3], const TileThread& tt, int (&lo)[3], int (&hi)[3]) {
   __shared__ int red[6][kTileThreads / 32];
   int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
 #pragma unroll
   for (int a = 0; a < kTilePts; ++a) {
-    if (!tt.valid_idx(a)) continue;
-    const int b1 = tt.x1(a) + (int)floorf(dd[a][0]) - 1;
-    const int b2 = tt.i2 + (int)floorf(dd[a][1]) - 1;
-    const int b3 = tt.i3 + (int)floorf(dd[a][2]) - 1;
-    mn[0] = min(mn[0], b1);
-    mx[0] = max(mx[0], b1);
-    mn[1] = min(mn[1], b2);
-    mx[1] = max(mx[1], b2);
-    mn[2] = min(mn[2], b3);
-    mx[2] = max(mx[2], b3);
+    const int b[3] = {tt.x1(a) + (int)floorf(dd[a][0]) - 1, tt.x2 + (int)floorf(dd[a][1]) - 1,
+                      tt.x3 + (int)floorf(dd[a][2]) - 1};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      mn[k] = min(mn[k], b[k]);
+      mx[k] = max(mx[k], b[k]);
+    }
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -175,45 +219,32 @@ CB_DEVICE void tile_bounds(const float (&dd)[kTilePts][3], const TileThread& tt,
   }
 }
 
-CB_DEVICE TileBox tile_box(const float (&dd)[kTilePts][3], const TileThread& tt, const Dims& d) {
-  int lo[3], hi[3];
-  tile_bounds(dd, tt, lo, hi);
-  return box_from_bounds(lo, hi, d);
-}
-
 // Per-tile box table of a displacement field: the tile's TileBox packed in two
-// int4, {lo1, lo2, lo3, e1 | e2 << 16}, {e3 | P << 16, Q, vol, within}.  It
-// depends on the displacement only, so one table serves every gather at that
-// characteristic (all time steps, all matvecs of a GN iterate).
+// int4, {lo1, lo2, lo3, fits}, {e1, e2, e3, Q}.  It depends on the displacement
+// only, so one table serves every gather at that characteristic (all time
+// steps, all matvecs of a GN iterate).
 CB_DEVICE void pack_box(const TileBox& bx, int4& a, int4& b) {
-  a = make_int4(bx.lo[0], bx.lo[1], bx.lo[2], (bx.e1 & 0xffff) | (bx.e2 << 16));
-  b = make_int4((bx.e3 & 0xffff) | (bx.P << 16), bx.Q, bx.vol, bx.within ? 1 : 0);
+  a = make_int4(bx.lo[0], bx.lo[1], bx.lo[2], bx.fits ? 1 : 0);
+  b = make_int4(bx.e1, bx.e2, bx.e3, bx.Q);
 }
 
-CB_DEVICE TileBox box_from_table(const int4* __restrict__ tab, const Dims&) {
+CB_DEVICE TileBox box_from_table(const int4* __restrict__ tab) {
   const int4 a = __ldg(tab + 2 * blockIdx.x), b = __ldg(tab + 2 * blockIdx.x + 1);
   TileBox bx;
   bx.lo[0] = a.x;
   bx.lo[1] = a.y;
   bx.lo[2] = a.z;
-  bx.e1 = a.w & 0xffff;
-  bx.e2 = a.w >> 16;
-  bx.e3 = b.x & 0xffff;
-  bx.P = b.x >> 16;
-  bx.Q = b.y;
-  bx.vol = b.z;
-  bx.within = b.w != 0;
+  bx.fits = a.w != 0;
+  bx.e1 = b.x;
+  bx.e2 = b.y;
+  bx.e3 = b.z;
+  bx.Q = b.w;
   return bx;
 }
 
-// ---- bulk box copies completing on an mbarrier ------------------------------
-// Count of tile gathers whose box copy did not complete within the wait limit
-// (the gather then skips its points); read by stage_timeouts().
+// ---- bounded wait (self-test of the device's failure counter) ---------------
+// Count of bounded waits that ran out; read by stage_timeouts().
 __device__ unsigned g_stage_timeouts = 0;
-
-// Wait limit of a box copy (ns of %globaltimer); the copies of one box take
-// microseconds.
-constexpr unsigned long long kStageWaitNs = 200000000ull;
 
 CB_DEVICE unsigned long long global_ns() {
   unsigned long long t;
@@ -221,8 +252,7 @@ CB_DEVICE unsigned long long global_ns() {
   return t;
 }
 CB_DEVICE void mbar_init(unsigned bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tfence.mbarrier_init.release.cluster;" ::"r"(bar)
-               : "memory");
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
 }
 // the barrier's one arrival, announcing the bytes its copies will deliver
 CB_DEVICE void mbar_arrive_expect(unsigned bar, unsigned bytes) {
@@ -239,67 +269,65 @@ CB_DEVICE bool mbar_test(unsigned bar, unsigned hint_ns) {
       : "memory");
   return ok != 0;
 }
-// Wait for phase 0 of the barrier for at most limit_ns; false on timeout.
-// Waiting threads sleep in try_wait (1 us at a time) instead of spinning.
-CB_DEVICE bool mbar_wait(unsigned bar, unsigned long long limit_ns) {
+// Wait for phase 0 of the barrier for at most limit_ns; a wait that runs out is
+// counted and reported as false.
+CB_DEVICE bool bounded_wait(unsigned bar, unsigned long long limit_ns) {
   if (mbar_test(bar, 1000u)) return true;
   const unsigned long long t0 = global_ns();
   while (!mbar_test(bar, 1000u))
-    if (global_ns() - t0 > limit_ns) return false;
+    if (global_ns() - t0 > limit_ns) {
+      atomicAdd(&g_stage_timeouts, 1u);
+      return false;
+    }
   return true;
 }
-CB_DEVICE void bulk_copy(unsigned dst, const float* src, unsigned bytes, unsigned bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
+
+// ---- box copies ---------------------------------------------------------------
+CB_DEVICE void copy16(unsigned dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// Bytes of a staged box (every copy of it lands on the barrier).
-CB_DEVICE unsigned box_bytes(const TileBox& bx) { return 4u * (unsigned)(bx.e1 * bx.e2 * bx.e3); }
-
-// Bulk copies of field f's box into the box at shared address sbase: row r of
-// the box (x1 plane r / e2, x2 row r % e2) by thread r (mod the CTA size).
-// Every source and destination is 16-byte aligned and every size a multiple
-// of 16 bytes: x3 starts on a multiple of 4 floats, N3 % 4 == 0, and P, Q are
-// multiples of 4.  (Issuing all rows from one warp instead ran 1.6 times
-// slower: the copies of a box must start from many threads at once.)
-CB_DEVICE void issue_box_bulk(unsigned sbase, const float* __restrict__ f, const TileBox& bx, const Dims& d,
-                              unsigned bar) {
-  const int rows = bx.e1 * bx.e2;
-  const int g3 = wrap_near(bx.lo[2], d.n3);
-  const int first = min(bx.e3, d.n3 - g3);  // floats before the x3 seam
-  const unsigned row = (unsigned)d.n3, plane = (unsigned)d.n2 * (unsigned)d.n3;
-  for (int r = threadIdx.x; r < rows; r += kTileThreads) {
-    const int l1 = small_div(r, bx.e2), l2 = r - l1 * bx.e2;
-    const int g1 = wrap_near(bx.lo[0] + l1, d.n1), g2 = wrap_near(bx.lo[1] + l2, d.n2);
-    const float* src = f + ((unsigned)g1 * plane + (unsigned)g2 * row);
-    const unsigned dst = sbase + 4u * (unsigned)(l1 * bx.Q + l2 * bx.P);
-    bulk_copy(dst, src + g3, 4u * (unsigned)first, bar);
-    if (first < bx.e3) bulk_copy(dst + 4u * (unsigned)first, src, 4u * (unsigned)(bx.e3 - first), bar);
+// Asynchronous copies of field f's box into the box at shared memory sb.  8
+// threads copy a row (chunks of 16 bytes), the CTA 32 rows at a time; the next
+// row of a thread is found without divisions.  Every chunk is 16-byte aligned
+// (x3 starts on a multiple of 4 floats, N3 % 4 == 0, P and Q are multiples of 4,
+// f is aligned) and none straddles the x3 seam.  (One bulk copy per row,
+// completing on an mbarrier, took 58 instructions a point: it is issued one lane
+// at a time, and the waiting warps spin.)
+CB_DEVICE void issue_box(float* sb, const float* __restrict__ f, const TileBox& bx, const Dims& d) {
+  constexpr int kRows = kTileThreads / 8;
+  const int lc = threadIdx.x & 7, nck = bx.e3 >> 2;
+  if (lc >= nck) return;
+  const int w3 = wrap_near(bx.lo[2], d.n3);
+  int g3 = w3 + 4 * lc, h3 = g3 + 32;  // rows of more than 32 floats: chunks 8 .. 11
+  g3 -= g3 >= d.n3 ? d.n3 : 0;
+  h3 -= h3 >= d.n3 ? d.n3 : 0;
+  const bool hi = lc + 8 < nck;
+  // row r = l1 e2 + l2; a step of kRows is s1 planes and s2 rows
+  const int r0 = threadIdx.x >> 3;
+  const int s1 = small_div(kRows, bx.e2), s2 = kRows - s1 * bx.e2;
+  int l1 = small_div(r0, bx.e2), l2 = r0 - l1 * bx.e2;
+  const int lo1 = wrap_near(bx.lo[0], d.n1), lo2 = wrap_near(bx.lo[1], d.n2);
+  unsigned dst = (unsigned)__cvta_generic_to_shared(sb) + 4u * (unsigned)(r0 * kPitch + 4 * lc);  // Q = e2 P
+  while (l1 < bx.e1) {
+    int g1 = lo1 + l1, g2 = lo2 + l2;
+    g1 -= g1 >= d.n1 ? d.n1 : 0;
+    g2 -= g2 >= d.n2 ? d.n2 : 0;
+    const float* src = f + (unsigned)(g1 * d.n2 + g2) * (unsigned)d.n3;
+    copy16(dst, src + g3);
+    if (hi) copy16(dst + 128u, src + h3);
+    dst += 4u * kRows * kPitch;
+    l1 += s1;
+    l2 += s2;
+    if (l2 >= bx.e2) {
+      l2 -= bx.e2;
+      ++l1;
+    }
   }
 }
 
-// Start the bulk copy of a staged box: barrier set up and armed with the box's
-// bytes by thread 0, published to the CTA, then the row copies.  Contains
-// __syncthreads: call from uniform control flow.
-CB_DEVICE void stage_box_start(unsigned sbase, const float* __restrict__ f, const TileBox& bx, const Dims& d,
-                               unsigned bar) {
-  if (threadIdx.x == 0) {
-    mbar_init(bar);
-    mbar_arrive_expect(bar, box_bytes(bx));
-  }
-  __syncthreads();
-  issue_box_bulk(sbase, f, bx, d, bar);
-}
-
-// Wait for the box; on timeout count it, wait once more for the copies still
-// in flight (bounded as well) and report false: the caller skips its points.
-CB_DEVICE bool stage_box_wait(unsigned bar, unsigned long long limit_ns) {
-  if (mbar_wait(bar, limit_ns)) return true;
-  if (threadIdx.x == 0) atomicAdd(&g_stage_timeouts, 1u);
-  mbar_wait(bar, limit_ns);
-  return false;
-}
+// This thread's copies have landed; a barrier then publishes the box.
+CB_DEVICE void copies_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // bf16 image field: the box is widened to FP32 while it is staged, with plain
 // loads and stores.  Warp w copies x1 planes w, w + 8, ...; its lanes cover
@@ -323,14 +351,14 @@ CB_DEVICE void issue_box(float* __restrict__ sb, const bf16* __restrict__ f, con
   constexpr int kWarps = kTileThreads / 32;
   for (int l1 = warp; l1 < bx.e1; l1 += kWarps) {
     const bf16* fp = fb + (unsigned)g1 * plane;
-    float* sp = sb + l1 * bx.Q + lr * bx.P + 4 * lc;
+    float* sp = sb + l1 * bx.Q + lr * kPitch + 4 * lc;
     int g2 = w2;
     for (int l2 = lr; l2 < bx.e2; l2 += rpi) {
       const uint2 raw = __ldg(reinterpret_cast<const uint2*>(fp + (unsigned)g2 * row));
       const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
       const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
       *reinterpret_cast<float4*>(sp) = make_float4(lo.x, lo.y, hi.x, hi.y);
-      sp += rpi * bx.P;
+      sp += rpi * kPitch;
       g2 += rpi;
       while (g2 >= d.n2) g2 -= d.n2;
     }
@@ -369,36 +397,10 @@ CB_DEVICE float gather_box(unsigned base, unsigned qb, const float (&w1)[4], con
   return acc;
 }
 
-// Shared-memory stencil of one point: tap (0,0,0) offset and weights.
-struct BoxPoint {
-  unsigned off;  // floats from the box origin
-  float w1[4], w2[4], w3[4];
-};
-
-CB_DEVICE BoxPoint box_point(const float (&dp)[3], int x1, const TileThread& tt, bool ok, const TileBox& bx) {
-  BoxPoint bp;
-  const float f1 = floorf(dp[0]), f2 = floorf(dp[1]), f3 = floorf(dp[2]);
-  lagrange4(dp[0] - f1, bp.w1);
-  lagrange4(dp[1] - f2, bp.w2);
-  lagrange4(dp[2] - f3, bp.w3);
-  const int o1 = ok ? x1 + (int)f1 - 1 - bx.lo[0] : 0;
-  const int o2 = ok ? tt.i2 + (int)f2 - 1 - bx.lo[1] : 0;
-  const int o3 = ok ? tt.i3 + (int)f3 - 1 - bx.lo[2] : 0;
-  bp.off = (unsigned)(o1 * bx.Q + o2 * bx.P + o3);
-  return bp;
-}
-
-CB_DEVICE float gather_staged(unsigned sb, const BoxPoint& bp, const TileBox& bx) {
-  const unsigned base = sb + bp.off * 4u;
-  const unsigned qb = (unsigned)bx.Q * 4u;
-  return bx.P == 32 ? gather_box<32>(base, qb, bp.w1, bp.w2, bp.w3) : gather_box<64>(base, qb, bp.w1, bp.w2, bp.w3);
-}
-
-// ---- two points per instruction: packed FP32 pairs (fma.rn.f32x2) ------------
-// The thread's points a and a+1 are gathered together: their weights and
-// partial sums live in 64-bit register pairs and every multiply-add of the
-// tensor product is one f32x2 instruction for both points (each lane an
-// ordinary round-to-nearest FP32 FMA, in the scalar code's order).
+// ---- packed FP32 pairs (fma.rn.f32x2) ------------------------------------------
+// Two multiply-adds per instruction, each lane an ordinary round-to-nearest
+// FP32 FMA.  The pairs are two x2 rows of a plane at one x3 column: their words
+// arrive by separate 32-bit loads, so pairing them costs nothing.
 typedef unsigned long long f32x2;
 
 CB_DEVICE f32x2 pk2(float a, float b) {
@@ -421,6 +423,7 @@ CB_DEVICE f32x2 mul2(f32x2 a, f32x2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+
 CB_DEVICE f32x2 dup2(float c) { return pk2(c, c); }
 
 // lagrange4 of two fractions at once (same Horner steps)
@@ -431,181 +434,292 @@ CB_DEVICE void lagrange4x2(f32x2 s, f32x2 (&w)[4]) {
   w[3] = mul2(s, fma2(mul2(s, s), dup2(1.f / 6.f), dup2(-1.f / 6.f)));
 }
 
-// Four consecutive floats at OFF from each of two addresses, weighted.
 template <int OFF>
-CB_DEVICE f32x2 row4x2(unsigned pa, unsigned pb, const f32x2 (&w)[4]) {
-  float a0, a1, a2, a3, b0, b1, b2, b3;
-  asm volatile(
-      "ld.shared.f32 %0, [%8+%10];\n\t"
-      "ld.shared.f32 %1, [%8+%11];\n\t"
-      "ld.shared.f32 %2, [%8+%12];\n\t"
-      "ld.shared.f32 %3, [%8+%13];\n\t"
-      "ld.shared.f32 %4, [%9+%10];\n\t"
-      "ld.shared.f32 %5, [%9+%11];\n\t"
-      "ld.shared.f32 %6, [%9+%12];\n\t"
-      "ld.shared.f32 %7, [%9+%13];\n"
-      : "=f"(a0), "=f"(a1), "=f"(a2), "=f"(a3), "=f"(b0), "=f"(b1), "=f"(b2), "=f"(b3)
-      : "r"(pa), "r"(pb), "n"(OFF), "n"(OFF + 4), "n"(OFF + 8), "n"(OFF + 12));
-  f32x2 r = mul2(w[0], pk2(a0, b0));
-  r = fma2(w[1], pk2(a1, b1), r);
-  r = fma2(w[2], pk2(a2, b2), r);
-  return fma2(w[3], pk2(a3, b3), r);
+CB_DEVICE float lds(unsigned addr) {
+  float x;
+  asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(x) : "r"(addr), "n"(OFF));
+  return x;
 }
 
-template <int P>
-CB_DEVICE f32x2 gather_box_x2(unsigned ba, unsigned bb, unsigned qb, const f32x2 (&w1)[4], const f32x2 (&w2)[4],
-                              const f32x2 (&w3)[4]) {
-  f32x2 acc = 0ull;
+// The first NC words of a row (byte offset OFF), and of the rows r and r + 1 as
+// pairs.
+template <int OFF, int NC>
+CB_DEVICE void row1(unsigned addr, float (&x)[NC]) {
+  x[0] = lds<OFF>(addr);
+  x[1] = lds<OFF + 4>(addr);
+  x[2] = lds<OFF + 8>(addr);
+  x[3] = lds<OFF + 12>(addr);
+  if constexpr (NC > 4) x[4] = lds<OFF + 16>(addr);
+}
+template <int OFF, int NC>
+CB_DEVICE void rows2(unsigned addr, f32x2 (&x)[NC]) {
+  float a[NC], b[NC];
+  row1<OFF>(addr, a);
+  row1<OFF + 4 * kPitch>(addr, b);
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const unsigned pa = ba + a * qb, pb = bb + a * qb;
-    f32x2 t = mul2(w2[0], row4x2<0>(pa, pb, w3));
-    t = fma2(w2[1], row4x2<P * 4>(pa, pb, w3), t);
-    t = fma2(w2[2], row4x2<P * 8>(pa, pb, w3), t);
-    t = fma2(w2[3], row4x2<P * 12>(pa, pb, w3), t);
-    acc = (a == 0) ? mul2(w1[0], t) : fma2(w1[a], t, acc);
-  }
-  return acc;
+  for (int c = 0; c < NC; ++c) x[c] = pk2(a[c], b[c]);
 }
 
-// Staged gather of the thread's points a and a+1: values (x, y).
-CB_DEVICE float2 gather_staged_pair(unsigned sb, const float (&da)[3], const float (&db)[3], int a,
-                                    const TileThread& tt, const TileBox& bx) {
-  float fa[3], fb[3];
-  int oa[3], ob[3];
-  const int xa[3] = {tt.x1(a), tt.i2, tt.i3}, xb[3] = {tt.x1(a + 1), tt.i2, tt.i3};
-  const bool okA = tt.valid_idx(a), okB = tt.valid_idx(a + 1);
+template <int NC>
+CB_DEVICE f32x2 row_sums(const f32x2 (&x)[NC], const f32x2 (&w3)[NC]) {
+  f32x2 t = mul2(w3[0], x[0]);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float la = floorf(da[k]), lb = floorf(db[k]);
-    fa[k] = da[k] - la;
-    fb[k] = db[k] - lb;
-    oa[k] = okA ? xa[k] + (int)la - 1 - bx.lo[k] : 0;
-    ob[k] = okB ? xb[k] + (int)lb - 1 - bx.lo[k] : 0;
-  }
-  f32x2 w1[4], w2[4], w3[4];
-  lagrange4x2(pk2(fa[0], fb[0]), w1);
-  lagrange4x2(pk2(fa[1], fb[1]), w2);
-  lagrange4x2(pk2(fa[2], fb[2]), w3);
-  const unsigned ba = sb + 4u * (unsigned)(oa[0] * bx.Q + oa[1] * bx.P + oa[2]);
-  const unsigned bb = sb + 4u * (unsigned)(ob[0] * bx.Q + ob[1] * bx.P + ob[2]);
-  const unsigned qb = (unsigned)bx.Q * 4u;
-  const f32x2 r = bx.P == 32 ? gather_box_x2<32>(ba, bb, qb, w1, w2, w3) : gather_box_x2<64>(ba, bb, qb, w1, w2, w3);
-  return upk2(r);
+  for (int c = 1; c < NC; ++c) t = fma2(w3[c], x[c], t);
+  return t;
 }
 
-// Tile gather of one field at the displacements Src loads; epi(tt, a, value)
-// consumes the value at the thread's point a.  sb holds kGatherBudget floats
-// (16-byte aligned).  Tiles whose box does not fit gather from global memory.
-// Several fields at one characteristic run as several CTAs (grid.z), each
-// reducing the same box: the extra displacement reads are L2 hits.
+// Weights of points A and B (fractions s, t): along x1, along x2 as row pairs,
+// along x3 duplicated.
+struct PairWeights {
+  float w1[2][4];
+  f32x2 w2[2][2], w3[2][4];
+  CB_DEVICE PairWeights(const float (&s)[3], const float (&t)[3]) {
+    f32x2 w[4];
+    float2 u[4];
+    lagrange4x2(pk2(s[0], t[0]), w);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      u[c] = upk2(w[c]);
+      w1[0][c] = u[c].x;
+      w1[1][c] = u[c].y;
+    }
+    lagrange4x2(pk2(s[1], t[1]), w);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) u[c] = upk2(w[c]);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      w2[0][c] = pk2(u[2 * c].x, u[2 * c + 1].x);
+      w2[1][c] = pk2(u[2 * c].y, u[2 * c + 1].y);
+    }
+    lagrange4x2(pk2(s[2], t[2]), w);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      u[c] = upk2(w[c]);
+      w3[0][c] = dup2(u[c].x);
+      w3[1][c] = dup2(u[c].y);
+    }
+  }
+};
+
+// Points A (planes 0..3 from base) and B (planes 1..4) in one pass over five
+// planes qb bytes apart; `last` is the address of plane 4 (any box address where
+// B is not wanted).  One row pair is live at a time.
+CB_DEVICE float2 gather_pair(unsigned base, unsigned qb, unsigned last, const PairWeights& w) {
+  float ra = 0.f, rb = 0.f;
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const unsigned pa = q < 4 ? base + q * qb : last;
+    f32x2 ta = 0ull, tb = 0ull;
+    {
+      f32x2 x[4];
+      rows2<0>(pa, x);
+      if (q < 4) ta = mul2(w.w2[0][0], row_sums(x, w.w3[0]));
+      if (q > 0) tb = mul2(w.w2[1][0], row_sums(x, w.w3[1]));
+    }
+    {
+      f32x2 x[4];
+      rows2<8 * kPitch>(pa, x);
+      if (q < 4) ta = fma2(w.w2[0][1], row_sums(x, w.w3[0]), ta);
+      if (q > 0) tb = fma2(w.w2[1][1], row_sums(x, w.w3[1]), tb);
+    }
+    if (q < 4) {
+      const float2 t = upk2(ta);
+      ra = fmaf(w.w1[0][q], t.x + t.y, ra);
+    }
+    if (q > 0) {
+      const float2 t = upk2(tb);
+      rb = fmaf(w.w1[1][q - 1], t.x + t.y, rb);
+    }
+  }
+  return make_float2(ra, rb);
+}
+
+// Fractions s of displacement dd and the shared address of the stencil's first
+// tap, `origin` being the address of the tap at floor(d) = 0.  Addresses
+// o1 Q + o2 P + o3 (o2 < ext2, o3 < P) are distinct for distinct taps.
+CB_DEVICE unsigned point_stencil(const float (&dd)[3], unsigned origin, unsigned qb, float (&s)[3]) {
+  const float f1 = floorf(dd[0]), f2 = floorf(dd[1]), f3 = floorf(dd[2]);
+  s[0] = dd[0] - f1;
+  s[1] = dd[1] - f2;
+  s[2] = dd[2] - f3;
+  return origin + (unsigned)(int)f1 * qb + (unsigned)(int)f2 * (4 * kPitch) + 4u * (unsigned)(int)f3;
+}
+
+// Address of the first tap of point (x1, x2, x3) at floor(d) = 0 (taken modulo
+// 2^32: it may lie outside the box).
+CB_DEVICE unsigned tap_origin(unsigned sb, int x1, int x2, int x3, const TileBox& bx) {
+  return sb + 4u * (unsigned)((x1 - 1 - bx.lo[0]) * bx.Q + (x2 - 1 - bx.lo[1]) * kPitch + (x3 - 1 - bx.lo[2]));
+}
+
+// Points of the tile that are gathered one by one.
+struct PointList {
+  unsigned short* id;  // 4 * thread + point
+  int* count;
+  CB_DEVICE void push(bool want, int point) const {
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    if (!m) return;
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(count, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (want) id[at] = (unsigned short)(kTilePts * threadIdx.x + point);
+  }
+};
+
+// Staged gather of the tile's points: epi(index, value, aux) for every point
+// inside the grid.  Contains __syncthreads: call from uniform control flow.
 template <class Src, class Epi>
-CB_DEVICE void tile_gather(float* sb, const Src& src, const float* __restrict__ f, const Dims& d, const Epi& epi) {
-  const TileThread tt = tile_thread(d);
-  // the box barrier is set up first: tile_box's own barriers publish it
-  __shared__ alignas(8) unsigned long long mbar;
-  const unsigned bar = (unsigned)__cvta_generic_to_shared(&mbar);
-  if (threadIdx.x == 0) mbar_init(bar);
-  float dd[kTilePts][3];
-  src.load(dd, tt, d);
-  const TileBox bx = tile_box(dd, tt, d);
-  if (bx.within && bx.vol <= kGatherBudget) {
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(sb);
-    // thread 0 arms the barrier while the copies start: bytes that land
-    // before the arrival take its transaction count below zero, and the
-    // phase cannot complete before the arrival
-    if (threadIdx.x == 0) mbar_arrive_expect(bar, box_bytes(bx));
-    issue_box_bulk(sbase, f, bx, d, bar);
-    if (!stage_box_wait(bar, kStageWaitNs)) return;
-    // two points per instruction (packed f32x2 pairs), as the table-driven gathers
+CB_DEVICE void gather_tile(unsigned sb, const PointList& list, const Src& src, const float (&dd)[kTilePts][3],
+                           const float (&aux)[kTilePts], const TileThread& tt, const TileBox& bx, const Dims& d,
+                           const TileGrid& tg, const Epi& epi) {
+  const unsigned qb = (unsigned)bx.Q * 4u;
+  const unsigned origin = tap_origin(sb, tt.x1_, tt.x2, tt.x3, bx);
 #pragma unroll
-    for (int a = 0; a < kTilePts; a += 2) {
-      const float2 r = gather_staged_pair(sbase, dd[a], dd[a + 1], a, tt, bx);
-      epi(tt, a, r.x);
-      epi(tt, a + 1, r.y);
-    }
-  } else {
-#pragma unroll
-    for (int a = 0; a < kTilePts; ++a) {
-      if (!tt.valid_idx(a)) continue;
-      Stencil st;
-      make_stencil(tt.x1(a), tt.i2, tt.i3, dd[a][0], dd[a][1], dd[a][2], d, st);
-      epi(tt, a, gather(f, st));
-    }
+  for (int a = 0; a < kTilePts; a += 2) {
+    float s[3], t[3];
+    const unsigned base = point_stencil(dd[a], origin + (unsigned)tt.step(a) * qb, qb, s);
+    const unsigned baseb = point_stencil(dd[a + 1], origin + (unsigned)tt.step(a + 1) * qb, qb, t);
+    const bool shared = baseb == base + qb;
+    list.push(tt.valid(a + 1) && !shared, a + 1);
+    const float2 r = gather_pair(base, qb, shared ? base + 4 * qb : base, PairWeights(s, t));
+    if (tt.valid(a)) epi(tt.idx(a), r.x, aux[a]);
+    if (shared && tt.valid(a + 1)) epi(tt.idx(a + 1), r.y, aux[a + 1]);
+  }
+  __syncthreads();
+  const int n = *list.count;
+  if (threadIdx.x >= n) return;
+  int t1, t2, t3;
+  tile_origin(tg, t1, t2, t3);
+  for (int i = threadIdx.x; i < n; i += kTileThreads) {
+    const int id = list.id[i];
+    int l1, l2, l3;
+    tile_local(id / kTilePts, l1, l2, l3);
+    const int x1 = t1 + l1 + plane_of(id % kTilePts), x2 = t2 + l2, x3 = t3 + l3;
+    const unsigned at = (unsigned)x1 * tt.plane + (unsigned)x2 * (unsigned)d.n3 + (unsigned)x3;
+    float de[3], s[3], w1[4], w2[4], w3[4];
+    src.at(de, at, d);
+    const float ae = epi.aux ? __ldg(epi.aux + at) : 0.f;
+    const unsigned base = point_stencil(de, tap_origin(sb, x1, x2, x3, bx), qb, s);
+    lagrange4(s[0], w1);
+    lagrange4(s[1], w2);
+    lagrange4(s[2], w3);
+    epi(at, gather_box<kPitch>(base, qb, w1, w2, w3), ae);
   }
 }
 
-// Tile gather of one field at a displacement field with a precomputed box
-// table: the box copy is issued first and the points' displacements (and the
-// epilogue's per-point operand epi.aux, when it has one) load while it is in
-// flight; epi(tt, a, value, aux_a) finishes point a.  T = bf16 stages an
-// image field synchronously (widened to FP32 on the way to shared memory).
-template <class Epi, class T = float>
-CB_DEVICE void tile_gather_tab(float* sb, const float* __restrict__ disp, const int4* __restrict__ tab,
-                               const T* __restrict__ f, const Dims& d, const Epi& epi) {
-  const TileBox bx = box_from_table(tab, d);
-  const bool staged = bx.within && bx.vol <= kGatherBudget;
-  __shared__ alignas(8) unsigned long long mbar;
-  const unsigned bar = (unsigned)__cvta_generic_to_shared(&mbar);
-  const unsigned sbase = (unsigned)__cvta_generic_to_shared(sb);
-  if (staged) {
-    if constexpr (std::is_same<T, float>::value) {
-      stage_box_start(sbase, f, bx, d, bar);
-    } else {
-      issue_box(sb, f, bx, d);  // bf16: widened to FP32 while staged (synchronous)
-    }
-  }
-  const TileThread tt = tile_thread(d);
-  float dd[kTilePts][3], aux[kTilePts];
-  const float* d2 = disp + d.n();
-  const float* d3 = d2 + d.n();
+// Global-memory gather of the thread's points (tiles whose box does not fit).
+template <class T, class Epi>
+CB_DEVICE void gather_unstaged(const T* __restrict__ f, const float (&dd)[kTilePts][3], const float (&aux)[kTilePts],
+                               const TileThread& tt, const Dims& d, const Epi& epi) {
 #pragma unroll
   for (int a = 0; a < kTilePts; ++a) {
-    const bool ok = tt.valid_idx(a);
-    const unsigned i = tt.idx(a);
-    dd[a][0] = ok ? __ldg(disp + i) : 0.f;
-    dd[a][1] = ok ? __ldg(d2 + i) : 0.f;
-    dd[a][2] = ok ? __ldg(d3 + i) : 0.f;
-    aux[a] = (ok && epi.aux) ? __ldg(epi.aux + i) : 0.f;
+    if (!tt.valid(a)) continue;
+    Stencil st;
+    make_stencil(tt.x1(a), tt.x2, tt.x3, dd[a][0], dd[a][1], dd[a][2], d, st);
+    epi(tt.idx(a), gather(f, st), aux[a]);
   }
-  if (staged) {
-    if constexpr (std::is_same<T, float>::value) {
-      if (!stage_box_wait(bar, kStageWaitNs)) return;
-    } else {
-      __syncthreads();
-    }
-#pragma unroll
-    for (int a = 0; a < kTilePts; a += 2) {
-      const float2 r = gather_staged_pair(sbase, dd[a], dd[a + 1], a, tt, bx);
-      epi(tt, a, r.x, aux[a]);
-      epi(tt, a + 1, r.y, aux[a + 1]);
-    }
-  } else {
-#pragma unroll
-    for (int a = 0; a < kTilePts; ++a) {
-      if (!tt.valid_idx(a)) continue;
-      Stencil st;
-      make_stencil(tt.x1(a), tt.i2, tt.i3, dd[a][0], dd[a][1], dd[a][2], d, st);
-      epi(tt, a, gather(f, st), aux[a]);
-    }
-  }
+}
+
+// Fields whose rows cannot be copied in 16-byte chunks (8 for bf16) gather from
+// global memory.
+template <class T>
+CB_DEVICE bool aligned_field(const T* f) {
+  return (reinterpret_cast<uintptr_t>(f) & (4 * sizeof(T) - 1)) == 0;
+}
+
+CB_DEVICE PointList point_list(float* sb, int* count) {
+  return PointList{reinterpret_cast<unsigned short*>(sb + kGatherBudget), count};
 }
 
 // Displacements of the tile's points from a displacement field (3 arrays n apart).
 struct DispSource {
   const float* ds;
-  CB_DEVICE void load(float (&dd)[kTilePts][3], const TileThread& tt, const Dims& d) const {
+  CB_DEVICE void at(float (&dd)[3], unsigned i, const Dims& d) const {
     const float* d2 = ds + d.n();
-    const float* d3 = d2 + d.n();
-#pragma unroll
-    for (int a = 0; a < kTilePts; ++a) {
-      const bool ok = tt.valid(a, d);
-      const unsigned i = tt.idx(a);
-      dd[a][0] = ok ? __ldg(ds + i) : 0.f;
-      dd[a][1] = ok ? __ldg(d2 + i) : 0.f;
-      dd[a][2] = ok ? __ldg(d3 + i) : 0.f;
-    }
+    dd[0] = __ldg(ds + i);
+    dd[1] = __ldg(d2 + i);
+    dd[2] = __ldg(d2 + d.n() + i);
   }
 };
+
+template <class Src>
+CB_DEVICE void load_points(const Src& src, float (&dd)[kTilePts][3], const TileThread& tt, const Dims& d) {
+#pragma unroll
+  for (int a = 0; a < kTilePts; ++a) src.at(dd[a], tt.idx(a), d);
+}
+
+// Tile gather of the fields f + k ff, k < nf, at the displacements of Src, one
+// after another: the displacements, their box and the tile set-up are shared.
+// tab (may be null) is the displacement's box table: with it the first copy is
+// issued before the displacements load; without it the CTA reduces its box
+// itself.  epi(k) is field k's epilogue, called as (index, value, aux) with
+// aux = epi(k).aux[index] (0 where it has none).  sb holds kGatherSmemBytes
+// (16-byte aligned).  A bf16 field is widened to FP32 while it is staged.
+template <class T, class Src, class MakeEpi>
+CB_DEVICE void tile_gather(float* sb, const Src& src, const int4* __restrict__ tab, const T* __restrict__ f,
+                           long long ff, int nf, const Dims& d, const TileGrid& tg, const MakeEpi& epi) {
+  __shared__ int listed[2];
+  const TileThread tt = tile_thread(d, tg);
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(sb);
+  float dd[kTilePts][3];
+  TileBox bx;
+  if (threadIdx.x == 0) listed[0] = 0;
+  if (tab) {
+    bx = box_from_table(tab);
+    if (bx.fits && aligned_field(f)) issue_box(sb, f, bx, d);
+    load_points(src, dd, tt, d);
+  } else {
+    load_points(src, dd, tt, d);
+    int lo[3], hi[3];
+    tile_bounds(dd, tt, lo, hi);
+    bx = box_from_bounds(lo, hi, d);
+    if (bx.fits && aligned_field(f)) issue_box(sb, f, bx, d);
+  }
+#pragma unroll 1
+  for (int k = 0; k < nf; ++k, f += ff) {
+    const auto e = epi(k);
+    const bool staged = bx.fits && aligned_field(f);
+    if (k) {
+      __syncthreads();  // field k - 1 is done with the box and its list
+      if (staged) issue_box(sb, f, bx, d);
+    }
+    float aux[kTilePts];
+#pragma unroll
+    for (int a = 0; a < kTilePts; ++a) aux[a] = e.aux ? __ldg(e.aux + tt.idx(a)) : 0.f;
+    if (threadIdx.x == 0) listed[(k + 1) & 1] = 0;  // the next field's
+    if (!staged) {
+      gather_unstaged(f, dd, aux, tt, d, e);
+      continue;
+    }
+    copies_landed();
+    __syncthreads();
+    // opaque per field: weights hoisted out of this loop would not fit in
+    // registers (here, after every load is issued: the statement waits for dd)
+#pragma unroll
+    for (int a = 0; a < kTilePts; ++a) asm volatile("" : "+f"(dd[a][0]), "+f"(dd[a][1]), "+f"(dd[a][2]));
+    gather_tile(sbase, point_list(sb, &listed[k & 1]), src, dd, aux, tt, bx, d, tg, e);
+  }
+}
+
+// The same for one field with a table (the time steps), without the loop's
+// state: 5% faster than tile_gather with nf = 1.
+template <class T, class Src, class Epi>
+CB_DEVICE void tile_step(float* sb, const Src& src, const int4* __restrict__ tab, const T* __restrict__ f,
+                         const Dims& d, const TileGrid& tg, const Epi& e) {
+  __shared__ int listed;
+  const TileBox bx = box_from_table(tab);
+  const bool staged = bx.fits && aligned_field(f);
+  if (staged) issue_box(sb, f, bx, d);
+  const TileThread tt = tile_thread(d, tg);
+  if (threadIdx.x == 0) listed = 0;
+  float dd[kTilePts][3], aux[kTilePts];
+  load_points(src, dd, tt, d);
+#pragma unroll
+  for (int a = 0; a < kTilePts; ++a) aux[a] = e.aux ? __ldg(e.aux + tt.idx(a)) : 0.f;
+  if (!staged) return gather_unstaged(f, dd, aux, tt, d, e);
+  copies_landed();
+  __syncthreads();
+  gather_tile((unsigned)__cvta_generic_to_shared(sb), point_list(sb, &listed), src, dd, aux, tt, bx, d, tg, e);
+}
 
 }  // namespace cb

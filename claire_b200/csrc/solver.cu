@@ -209,14 +209,14 @@ long long Solver::estimate_bytes(const claire_b200_opts& o, int B) {
   return bytes;
 }
 
-// A tile gather whose box copy ran out of its bounded wait skipped its tile
-// (sl_tile.cuh); report it once, at the next GN-iteration boundary.
+// A bounded device wait ran out (sl_tile.cuh); report it once, at the next
+// GN-iteration boundary.
 int Solver::check_stage() {
   unsigned long long t = 0;
   if (stage_timeouts(&t, stream)) return CB_ERR_CUDA;
   if (t <= stage_seen) return 0;
   stage_seen = t;
-  err = "a tile gather's shared-memory box copy did not complete within its wait limit";
+  err = "a bounded device wait did not complete within its limit";
   return CB_ERR_CUDA;
 }
 
