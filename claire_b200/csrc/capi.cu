@@ -899,24 +899,23 @@ int claire_b200_fft_div(const float* v, float* dout, const int nx[3], void* stre
   return CB_OK;
 }
 
-// scratch for a 3-field spectral op: spectrum, params, partials, result slot
+// scratch for a spectral op of nf fields: spectrum and, with nparts, reduction
+// partials and their result
 struct Scratch {
   float2* spec = nullptr;
-  SpecParams* params = nullptr;
   double* partials = nullptr;
   double* result = nullptr;
   cudaStream_t s = nullptr;
-  int alloc(const Dims& d, int nparts, cudaStream_t st) {
+  int alloc(const Dims& d, int nf, int nparts, cudaStream_t st) {
     s = st;
-    if (cudaMallocAsync((void**)&spec, sizeof(float2) * 3 * d.nc(), s) != cudaSuccess) return CB_ERR_ALLOC;
-    if (cudaMallocAsync((void**)&params, sizeof(SpecParams), s) != cudaSuccess) return CB_ERR_ALLOC;
+    if (cudaMallocAsync((void**)&spec, sizeof(float2) * nf * d.nc(), s) != cudaSuccess) return CB_ERR_ALLOC;
+    if (!nparts) return CB_OK;
     if (cudaMallocAsync((void**)&partials, sizeof(double) * (nparts + 1), s) != cudaSuccess) return CB_ERR_ALLOC;
     result = partials + nparts;
     return CB_OK;
   }
   ~Scratch() {
     if (spec) cudaFreeAsync(spec, s);
-    if (params) cudaFreeAsync(params, s);
     if (partials) cudaFreeAsync(partials, s);
   }
 };
@@ -935,13 +934,12 @@ static SpecParams make_params(const Dims& d, int regnorm, const double* beta, do
 static int spectral3(const float* in, float* out, const Dims& d, int op, const SpecParams& hp, int epi,
                      double* sumsq, cudaStream_t st) {
   Scratch sc;
-  const int np = std::max(1, c2r_partials(d, 3));
-  int e = sc.alloc(d, np, st);
+  const int np = epi == EPI_SUMSQ ? std::max(1, c2r_partials(d, 3)) : 0;
+  int e = sc.alloc(d, 3, np, st);
   if (e) return e;
-  if (cudaMemcpyAsync(sc.params, &hp, sizeof(SpecParams), cudaMemcpyHostToDevice, st) != cudaSuccess) return CB_ERR_CUDA;
   const long long n = d.n(), nc = d.nc();
   e = launch_r2c3d(in, 0, n, sc.spec, 0, 3, 1, d, nullptr, st);
-  if (!e) e = launch_pencil(sc.spec, 0, 1, d, op, sc.params, 3, 3, nullptr, st);
+  if (!e) e = launch_pencil(sc.spec, 0, 1, d, op, nullptr, 3, 3, nullptr, st, &hp);
   if (!e) e = launch_c2r3d(sc.spec, 0, out, 0, n, 3, 1, d, epi, nullptr, sc.partials, np, nullptr, st);
   if (!e && epi == EPI_SUMSQ) e = launch_finalize(sc.partials, np, np, sc.result, 1, 1.0, false, st);
   note_launches(6);
@@ -1036,14 +1034,13 @@ int claire_b200_smooth(const float* f, float* out, const int nx[3], const double
   Dims d{nx[0], nx[1], nx[2]};
   cudaStream_t st = (cudaStream_t)stream;
   Scratch sc;
-  int e = sc.alloc(d, 1, st);
+  int e = sc.alloc(d, 1, 0, st);
   if (e) return e;
   SpecParams p = make_params(d, 0, nullptr, 0.0);
   for (int k = 0; k < 3; ++k) p.sigma[k] = (float)sigma[k];
-  if (cudaMemcpyAsync(sc.params, &p, sizeof(SpecParams), cudaMemcpyHostToDevice, st) != cudaSuccess) return CB_ERR_CUDA;
   const long long n = d.n();
   e = launch_r2c3d(f, 0, n, sc.spec, 0, 1, 1, d, nullptr, st);
-  if (!e) e = launch_pencil(sc.spec, 0, 1, d, OP_GAUSS, sc.params, 1, 1, nullptr, st);
+  if (!e) e = launch_pencil(sc.spec, 0, 1, d, OP_GAUSS, nullptr, 1, 1, nullptr, st, &p);
   if (!e) e = launch_c2r3d(sc.spec, 0, out, 0, n, 1, 1, d, EPI_STORE, nullptr, nullptr, 0, nullptr, st);
   note_launches(5);
   return cuda_status(e);

@@ -498,7 +498,7 @@ struct DiagSymbol {
 template <int N, int V, bool DIAG>
 __global__ void __launch_bounds__(ColCfg<N, V>::T, (DIAG ? (ColCfg<N, V>::R1 > 12 ? 768 : 1024) : 512) / ColCfg<N, V>::T)
     k_pencil1(float2* __restrict__ spec, long long pstr, long long fstr, int nf, Dims d, int op, float s,
-              const SpecParams* __restrict__ params, const float2* __restrict__ twg,
+              const SpecParams* __restrict__ params, SpecParams one, const float2* __restrict__ twg,
               const int* __restrict__ active) {
   using F = ColCfg<N, V>;
   constexpr int C = F::C, R0 = F::R0, R1 = F::R1, STEP = F::T / C;
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(ColCfg<N, V>::T, (DIAG ? (ColCfg<N, V>::R1 > 1
   float2* col = spec + blockIdx.z * pstr + blockIdx.y * fstr + (ok ? g : 0);
   float* sig = reinterpret_cast<float*>(tw + N);
   load_twiddles<N, F::T>(tw, twg);
-  const SpecParams q = params[blockIdx.z];
+  const SpecParams q = params ? params[blockIdx.z] : one;
   const ColumnK ck = column_k(g / n3h, g % n3h, d);
   if constexpr (DIAG) {
     const DiagSymbol sym(op, q, s);
@@ -569,7 +569,7 @@ template <int N, int V>
 __global__ void __launch_bounds__(ColCfg<N, V>::T, 512 / ColCfg<N, V>::T) k_pencil3(float2* __restrict__ spec, long long pstr,
                                                               long long fstr, Dims d, int op, float s,
                                                               const SpecParams* __restrict__ params,
-                                                              const float2* __restrict__ twg,
+                                                              SpecParams one, const float2* __restrict__ twg,
                                                               const int* __restrict__ active) {
   using F = ColCfg<N, V>;
   constexpr int C = F::C, R0 = F::R0, R1 = F::R1;
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(ColCfg<N, V>::T, 512 / ColCfg<N, V>::T) k_penc
                            [&](int k0, float2 v) { S[(k0 * R1 + j) * C + c] = v; });
   }
   __syncthreads();
-  const SpecParams q = params[blockIdx.z];
+  const SpecParams q = params ? params[blockIdx.z] : one;
   const ColumnK ck = column_k(g / n3h, g % n3h, d);
   for (int k0 = u0; k0 < R0; k0 += F::T / C) {
     float2 v[3][R1];
@@ -919,7 +919,8 @@ static int cols_impl(float2* data, long long pstr, long long fstr, int ncols, in
 
 template <int N, int V>
 static int pencil_impl(float2* spec, long long sp, long long fstr, int nprob, const Dims& d, int op,
-                       const SpecParams* params, int nin, int nout, const int* active, cudaStream_t s) {
+                       const SpecParams* params, const SpecParams& one, int nin, int nout, const int* active,
+                       cudaStream_t s) {
   const float2* tw = twiddles(N);
   if (!tw) return (int)cudaErrorMemoryAllocation;
   const int ncols = d.n2 * (d.n3 / 2 + 1);
@@ -937,13 +938,13 @@ static int pencil_impl(float2* spec, long long sp, long long fstr, int nprob, co
   int e = 0;
   if (coupled) {
     if ((e = set_smem(k_pencil3<N, V>, sm))) return e;
-    k_pencil3<N, V><<<grid, T, sm, s>>>(spec, sp, fstr, d, op, scale, params, tw, active);
+    k_pencil3<N, V><<<grid, T, sm, s>>>(spec, sp, fstr, d, op, scale, params, one, tw, active);
   } else if (diag) {
     if ((e = set_smem(k_pencil1<N, V, true>, sm))) return e;
-    k_pencil1<N, V, true><<<grid, T, sm, s>>>(spec, sp, fstr, shared ? nin : 1, d, op, scale, params, tw, active);
+    k_pencil1<N, V, true><<<grid, T, sm, s>>>(spec, sp, fstr, shared ? nin : 1, d, op, scale, params, one, tw, active);
   } else {
     if ((e = set_smem(k_pencil1<N, V, false>, sm))) return e;
-    k_pencil1<N, V, false><<<grid, T, sm, s>>>(spec, sp, fstr, 1, d, op, scale, params, tw, active);
+    k_pencil1<N, V, false><<<grid, T, sm, s>>>(spec, sp, fstr, 1, d, op, scale, params, one, tw, active);
   }
   return (int)cudaGetLastError();
 }
@@ -970,10 +971,12 @@ int launch_r2c3d(const float* in, long long ip, long long ifs, float2* spec, lon
 }
 
 int launch_pencil(float2* spec, long long sp, int nprob, const Dims& d, int op,
-                  const SpecParams* dparams, int nin, int nout, const int* active, cudaStream_t s) {
-  if (!axes_supported(d)) return (int)cudaErrorInvalidValue;
+                  const SpecParams* dparams, int nin, int nout, const int* active, cudaStream_t s,
+                  const SpecParams* one) {
+  if (!axes_supported(d) || (!dparams && !one)) return (int)cudaErrorInvalidValue;
+  const SpecParams q = one ? *one : SpecParams{};
   int e = 0;
-  CB_DISPATCH_NV_COL(d.n1, e = (pencil_impl<NN, VV>(spec, sp, d.nc(), nprob, d, op, dparams, nin, nout, active, s)));
+  CB_DISPATCH_NV_COL(d.n1, e = (pencil_impl<NN, VV>(spec, sp, d.nc(), nprob, d, op, dparams, q, nin, nout, active, s)));
   return e;
 }
 
@@ -1137,7 +1140,7 @@ static int spectral3_explicit_impl(const float* in, float* out, float2* spec, co
   const size_t sm = col_smem<N, V>(1);
   k_cols<N, false, V><<<cols, T, sm, s>>>(spec, 0, nc, ncx2, n3h, (long long)d.n2 * n3h, n3h, tw, nullptr);
   k_pencil1<N, V, true><<<pen, T, col_smem<N, V>(1, true), s>>>(
-      spec, 0, nc, 3, d, op, 1.f / (float)((double)d.n1 * d.n2 * d.n3), params, tw, nullptr);
+      spec, 0, nc, 3, d, op, 1.f / (float)((double)d.n1 * d.n2 * d.n3), params, SpecParams{}, tw, nullptr);
   k_cols<N, true, V><<<cols, T, sm, s>>>(spec, 0, nc, ncx2, n3h, (long long)d.n2 * n3h, n3h, tw, nullptr);
   k_c2r_rows<N, V><<<rows, RowCfg<N, V>::T, RowCfg<N, V>::smem, s>>>(spec, 0, nc, out, 0, n, nrows, tw, EPI_STORE, nullptr,
                                                            nullptr, 0, nullptr, nullptr);

@@ -46,9 +46,12 @@ struct Batch {
 // Forward r2c of nf real fields: in[p*ip + f*ifs] -> spec[p*sp + f*nc].
 int launch_r2c3d(const float* in, long long ip, long long ifs, float2* spec, long long sp, int nf,
                  int nprob, const Dims& d, const int* active, cudaStream_t s);
-// Apply op in the x1 pass (in place on spec, nin fields in, nout out).
+// Apply op in the x1 pass (in place on spec, nin fields in, nout out).  The
+// problems' parameters come from device memory, or (dparams null) all from the
+// host's *one, which travels as a kernel argument.
 int launch_pencil(float2* spec, long long sp, int nprob, const Dims& d, int op,
-                  const SpecParams* dparams, int nin, int nout, const int* active, cudaStream_t s);
+                  const SpecParams* dparams, int nin, int nout, const int* active, cudaStream_t s,
+                  const SpecParams* one = nullptr);
 // Inverse c2r of nf fields with epilogue: out[p*op + f*ofs] = alpha[p]*x (+ out) or sumsq.
 int launch_c2r3d(float2* spec, long long sp, float* out, long long op_, long long ofs, int nf,
                  int nprob, const Dims& d, int epi, const float* alpha, double* partials, int nparts,
