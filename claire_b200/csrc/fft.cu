@@ -131,7 +131,7 @@ CB_DEVICE void rows_a(const float* __restrict__ ra, bool ok, int p, int j, float
 }
 
 // Inverse A butterfly and the epilogue: value e of row a / b is al times the
-// real / imaginary part; stored, added to dst, or squared and summed
+// real / imaginary part; stored, added to dst or to `oth`, or squared and summed
 // (returned), with the product with `oth` summed for the dot epilogues.  Old
 // values of a group of elements are loaded before any of them is stored.
 template <class F>
@@ -160,14 +160,15 @@ CB_DEVICE double rows_out(float* __restrict__ da, const float* __restrict__ oa, 
     }
     return acc;
   }
-  const bool add = (epi == EPI_ADD || epi == EPI_ADD_DOT), dot = epi != EPI_ADD;
+  const bool add = epi != EPI_STORE_DOT, dot = epi == EPI_STORE_DOT || epi == EPI_ADD_DOT;
+  const float* src = epi == EPI_SUM ? oa : da;
 #pragma unroll
   for (int r0 = 0; r0 < R0; r0 += G) {
     float2 old[G], oth[G];
 #pragma unroll
     for (int i = 0; i < G; ++i) {
       const int e = j + R1 * (r0 + i);
-      old[i] = add ? make_float2(da[e], da[N + e]) : make_float2(0.f, 0.f);
+      old[i] = add ? make_float2(src[e], src[N + e]) : make_float2(0.f, 0.f);
       oth[i] = dot ? make_float2(oa[e], oa[N + e]) : make_float2(0.f, 0.f);
     }
 #pragma unroll
@@ -1030,7 +1031,7 @@ int c2r_partials(const Dims& d, int nf, bool any_variant) {
 int launch_c2r3d(float2* spec, long long sp, float* out, long long op_, long long ofs, int nf,
                  int nprob, const Dims& d, int epi, const float* alpha, double* partials, int nparts,
                  const int* active, cudaStream_t s, const float* other) {
-  if ((epi == EPI_STORE_DOT || epi == EPI_ADD_DOT) && !other) return (int)cudaErrorInvalidValue;
+  if ((epi == EPI_STORE_DOT || epi == EPI_ADD_DOT || epi == EPI_SUM) && !other) return (int)cudaErrorInvalidValue;
   if (!axes_supported(d)) return (int)cudaErrorInvalidValue;
   const long long nc = d.nc();
   const int n3h = d.n3 / 2 + 1;

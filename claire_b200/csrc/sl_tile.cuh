@@ -441,7 +441,7 @@ CB_DEVICE float lds(unsigned addr) {
   return x;
 }
 
-// The first NC words of a row (byte offset OFF), and of the rows r and r + 1 as
+// The first NC words of a row (byte offset OFF), and of the rows r and r + 2 as
 // pairs.
 template <int OFF, int NC>
 CB_DEVICE void row1(unsigned addr, float (&x)[NC]) {
@@ -455,7 +455,7 @@ template <int OFF, int NC>
 CB_DEVICE void rows2(unsigned addr, f32x2 (&x)[NC]) {
   float a[NC], b[NC];
   row1<OFF>(addr, a);
-  row1<OFF + 4 * kPitch>(addr, b);
+  row1<OFF + 8 * kPitch>(addr, b);
 #pragma unroll
   for (int c = 0; c < NC; ++c) x[c] = pk2(a[c], b[c]);
 }
@@ -468,8 +468,9 @@ CB_DEVICE f32x2 row_sums(const f32x2 (&x)[NC], const f32x2 (&w3)[NC]) {
   return t;
 }
 
-// Weights of points A and B (fractions s, t): along x1, along x2 as row pairs,
-// along x3 duplicated.
+// Weights of points A and B (fractions s, t): along x1, along x2 as row pairs
+// (r, r + 2), so that a sum runs over neighbouring rows before the two halves
+// meet, along x3 duplicated.
 struct PairWeights {
   float w1[2][4];
   f32x2 w2[2][2], w3[2][4];
@@ -488,8 +489,8 @@ struct PairWeights {
     for (int c = 0; c < 4; ++c) u[c] = upk2(w[c]);
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      w2[0][c] = pk2(u[2 * c].x, u[2 * c + 1].x);
-      w2[1][c] = pk2(u[2 * c].y, u[2 * c + 1].y);
+      w2[0][c] = pk2(u[c].x, u[c + 2].x);
+      w2[1][c] = pk2(u[c].y, u[c + 2].y);
     }
     lagrange4x2(pk2(s[2], t[2]), w);
 #pragma unroll
@@ -518,7 +519,7 @@ CB_DEVICE float2 gather_pair(unsigned base, unsigned qb, unsigned last, const Pa
     }
     {
       f32x2 x[4];
-      rows2<8 * kPitch>(pa, x);
+      rows2<4 * kPitch>(pa, x);
       if (q < 4) ta = fma2(w.w2[0][1], row_sums(x, w.w3[0]), ta);
       if (q > 0) tb = fma2(w.w2[1][1], row_sums(x, w.w3[1]), tb);
     }

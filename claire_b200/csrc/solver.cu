@@ -240,8 +240,9 @@ int Solver::init(const claire_b200_opts& o, int Bn) {
     // CLAIRE_B200_GRAPHS=0 runs PCG iterations as direct launches
     const char* ge = std::getenv("CLAIRE_B200_GRAPHS");
     graphs = !(ge && ge[0] == '0');
+    // CLAIRE_B200_FUSED_DOTS=0 sums the PCG's dots in their own passes
     const char* fd = std::getenv("CLAIRE_B200_FUSED_DOTS");
-    fused_dots = fd && fd[0] == '1';
+    fused_dots = !(fd && fd[0] == '0');
     const char* rr = std::getenv("CLAIRE_B200_REG_RECURRENCE");
     reg_rec_enabled = !(rr && rr[0] == '0');
   }
@@ -806,10 +807,10 @@ int Solver::objective_at(const float* vel, const std::vector<int>& sel) {
 // ---------------------------------------------------------------------------
 // spectral building blocks
 // ---------------------------------------------------------------------------
-// out = F^-1(symbol F(vin)) with epilogue epi; with dot_with, out . dot_with
+// out = F^-1(symbol F(vin)) with epilogue epi (EPI_SUM: plus addend); with dot_with, out . dot_with
 // (FP64) lands in slot dot_slot (the inverse transform's epilogue sums it).
 int Solver::reg_op(const float* vin, float* out, int op, int epi, const int* act, const float* dot_with,
-                   int dot_slot) {
+                   int dot_slot, const float* addend) {
   CB_TRY(launch_r2c3d(vin, 3 * n, n, spec, 3 * nc, 3, B, d, act, stream));
   CB_TRY(launch_pencil(spec, 3 * nc, B, d, op, dparams, 3, 3, act, stream));
   if (dot_with && fused_dots) {
@@ -825,7 +826,7 @@ int Solver::reg_op(const float* vin, float* out, int op, int epi, const int* act
     note_launches(5);
     return dot(out, 3 * n, dot_with, 3 * n, 3 * n, dot_slot, act);
   }
-  CB_TRY(launch_c2r3d(spec, 3 * nc, out, 3 * n, n, 3, B, d, epi, nullptr, nullptr, 0, act, stream));
+  CB_TRY(launch_c2r3d(spec, 3 * nc, out, 3 * n, n, 3, B, d, epi, nullptr, nullptr, 0, act, stream, addend));
   note_launches(5);
   return 0;
 }
@@ -864,16 +865,15 @@ int Solver::adjoint_sweep(float* bout, const int* act, double hscale) {
     CB_TRY(prof_mark(CB_PROF_ADJOINT_STEP));
   }
   const bool proj = opts.model != CB_MODEL_COMPRESSIBLE;
-  CB_TRY(launch_body_force(lamh, PL, gm, PGM, bout, 3 * n, nt, ht, proj ? 1.f : (float)hfac, B, n, act, stream));
+  // the projection is linear: hd is applied here, where it costs no pass
+  CB_TRY(launch_body_force(lamh, PL, gm, PGM, bout, 3 * n, nt, ht, (float)hfac, B, n, act, stream));
   note_launches(nt + 1);
   if (proj) {
     CB_TRY(launch_r2c3d(bout, 3 * n, n, spec, 3 * nc, 3, B, d, act, stream));
     CB_TRY(launch_pencil(spec, 3 * nc, B, d, opts.model == CB_MODEL_STOKES ? OP_LERAY : OP_LERAY_RELAXED, dparams,
                          3, 3, act, stream));
     CB_TRY(launch_c2r3d(spec, 3 * nc, bout, 3 * n, n, 3, B, d, EPI_ADD, nullptr, nullptr, 0, act, stream));
-    CB_TRY(launch_lincomb(bout, 3 * n, bout, 3 * n, nullptr, hfac, nullptr, 0, nullptr, 0.0, 3 * n, B, act,
-                          stream));
-    note_launches(6);
+    note_launches(5);
   }
   return 0;
 }
@@ -890,10 +890,7 @@ int Solver::finish_with_reg(const float* vin, float* out, const int* act, const 
     CB_TRY(adjoint_sweep(bfo, act));
     if (norec_act) {
       if (proj) {
-        CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_STORE, norec_act));
-        CB_TRY(launch_lincomb(out, 3 * n, out, 3 * n, nullptr, 1.0, bf, 3 * n, nullptr, 1.0, 3 * n, B, norec_act,
-                              stream));
-        note_launches(1);
+        CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_SUM, norec_act, nullptr, -1, bf));
         if (dot_with) CB_TRY(dot(out, 3 * n, dot_with, 3 * n, 3 * n, dot_slot, norec_act));
       } else {
         CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_ADD, norec_act, dot_with, dot_slot));
@@ -917,9 +914,7 @@ int Solver::finish_with_reg(const float* vin, float* out, const int* act, const 
     return 0;
   }
   CB_TRY(adjoint_sweep(bf, act));
-  CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_STORE, act));
-  CB_TRY(launch_lincomb(out, 3 * n, out, 3 * n, nullptr, 1.0, bf, 3 * n, nullptr, 1.0, 3 * n, B, act, stream));
-  note_launches(1);
+  CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_SUM, act, nullptr, -1, bf));
   if (dot_with) CB_TRY(dot(out, 3 * n, dot_with, 3 * n, 3 * n, dot_slot, act));
   return 0;
 }

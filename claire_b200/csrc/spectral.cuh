@@ -31,10 +31,10 @@ struct SpecParams {
   float sigma[3];             // Gaussian width in grid cells
 };
 
-// Epilogue of the inverse row pass.
-// Epilogues of the inverse transforms: store, accumulate, sum of squares, or
-// store / accumulate and sum out * other (FP64 partials, c2r only).
-enum Epi : int { EPI_STORE = 0, EPI_ADD = 1, EPI_SUMSQ = 2, EPI_STORE_DOT = 3, EPI_ADD_DOT = 4 };
+// Epilogues of the inverse transforms: store, accumulate, sum of squares, and
+// (c2r only) store / accumulate and sum out * other (FP64 partials), or store
+// other + value.
+enum Epi : int { EPI_STORE = 0, EPI_ADD = 1, EPI_SUMSQ = 2, EPI_STORE_DOT = 3, EPI_ADD_DOT = 4, EPI_SUM = 5 };
 
 struct Batch {
   int nprob;              // problems in the launch
