@@ -21,8 +21,8 @@
 // points one per thread.
 //
 // Shared-memory layout of a box: x3 rows of pitch P = 48 floats (16 mod 32: the 2
-// rows of a warp use opposite halves of the bank space), x1 planes of stride
-// Q = ext2 * P.  Every shared-memory index is inside the box by construction:
+// rows of a warp use opposite halves of the bank space; 32 where only that
+// fits), x1 planes of stride Q = ext2 * P.  Every shared-memory index is inside the box by construction:
 // each point's taps lie in [i + floor(d) - 1, i + floor(d) + 2] and the box spans
 // the min / max of exactly those values over the tile's points; points outside
 // the grid (partial tiles) repeat the last point inside and are never stored.
@@ -31,10 +31,9 @@
 // one another's copies with their gathers.
 //
 // Measured in situ, 8 problems of 128^3, all launches of a solve's first two
-// Gauss-Newton iterations: adjoint steps 161 us (173 with a stencil per point,
-// 32-bit loads of 64 words a point and a bulk copy per box row), incremental
-// steps 153 (162), state steps 181 (205), the 24 cached gradient fields 4.08 ms
-// (4.61), characteristics 0.61 ms (0.72).
+// Gauss-Newton iterations: adjoint steps 159 us (173 with a stencil per point,
+// 64 words a point and a bulk copy per box row), incremental steps 156 (162), the
+// 24 cached gradient fields 4.05 ms (4.61), characteristics 0.62 ms (0.72).
 #pragma once
 
 #include <climits>
@@ -84,7 +83,8 @@ struct TileGrid {
   unsigned nb2, nb3, m2, m3;
   __host__ __device__ explicit TileGrid(const Dims& d)
       : nb2((d.n2 + kT2 - 1) / kT2), nb3((d.n3 + kT3 - 1) / kT3),
-        m2(nb2 == 1 ? 0u : (unsigned)((1ull << 32) / nb2) + 1u), m3(nb3 == 1 ? 0u : (unsigned)((1ull << 32) / nb3) + 1u) {}
+        m2(nb2 == 1 ? 0u : (unsigned)((1ull << 32) / nb2) + 1u),
+        m3(nb3 == 1 ? 0u : (unsigned)((1ull << 32) / nb3) + 1u) {}
 };
 
 CB_DEVICE unsigned tile_div(unsigned t, unsigned nb, unsigned m) {
@@ -146,12 +146,15 @@ CB_DEVICE TileThread tile_thread(const Dims& d, const TileGrid& tg) {
   return tt;
 }
 
-constexpr int kPitch = 48;  // x3 row pitch of a staged box (floats, 16 mod 32 banks)
+// x3 row pitches of a staged box: 48 floats (16 mod 32 banks), or 32 where only
+// that fits (strong maps; the two rows of a warp then share their banks, which
+// is far cheaper than gathering from global memory)
+constexpr int kPitch = 48, kPitchTight = 32;
 
 struct TileBox {
   int lo[3];
   int e1, e2, e3;  // extents (e3 in whole 16-byte chunks)
-  int Q;           // x1 plane stride (floats)
+  int P, Q;        // x3 row pitch, x1 plane stride (floats)
   bool fits;       // copyable (one wrap per axis, whole chunks) and within budget
 };
 
@@ -176,9 +179,10 @@ CB_DEVICE TileBox box_from_bounds(const int (&lo)[3], const int (&hi)[3], const 
   bx.lo[2] = lo3a;
   bx.e1 = ext[0];
   bx.e2 = ext[1];
-  bx.Q = bx.e2 * kPitch;
-  bx.fits = fits && bx.e3 <= d.n3 && bx.e3 <= kPitch && (d.n3 & 3) == 0 &&
-            (long long)bx.e1 * bx.Q <= kGatherBudget;
+  const long long rows = (long long)bx.e1 * bx.e2;
+  bx.P = bx.e3 <= kPitch && rows * kPitch <= kGatherBudget ? kPitch : kPitchTight;
+  bx.Q = bx.e2 * bx.P;
+  bx.fits = fits && bx.e3 <= d.n3 && bx.e3 <= bx.P && (d.n3 & 3) == 0 && rows * bx.P <= kGatherBudget;
   return bx;
 }
 
@@ -220,11 +224,11 @@ CB_DEVICE void tile_bounds(const float (&dd)[kTilePts][3], const TileThread& tt,
 }
 
 // Per-tile box table of a displacement field: the tile's TileBox packed in two
-// int4, {lo1, lo2, lo3, fits}, {e1, e2, e3, Q}.  It depends on the displacement
+// int4, {lo1, lo2, lo3, fits ? P : 0}, {e1, e2, e3, Q}.  It depends on the displacement
 // only, so one table serves every gather at that characteristic (all time
 // steps, all matvecs of a GN iterate).
 CB_DEVICE void pack_box(const TileBox& bx, int4& a, int4& b) {
-  a = make_int4(bx.lo[0], bx.lo[1], bx.lo[2], bx.fits ? 1 : 0);
+  a = make_int4(bx.lo[0], bx.lo[1], bx.lo[2], bx.fits ? bx.P : 0);
   b = make_int4(bx.e1, bx.e2, bx.e3, bx.Q);
 }
 
@@ -235,6 +239,7 @@ CB_DEVICE TileBox box_from_table(const int4* __restrict__ tab) {
   bx.lo[1] = a.y;
   bx.lo[2] = a.z;
   bx.fits = a.w != 0;
+  bx.P = a.w;
   bx.e1 = b.x;
   bx.e2 = b.y;
   bx.e3 = b.z;
@@ -308,7 +313,7 @@ CB_DEVICE void issue_box(float* sb, const float* __restrict__ f, const TileBox& 
   const int s1 = small_div(kRows, bx.e2), s2 = kRows - s1 * bx.e2;
   int l1 = small_div(r0, bx.e2), l2 = r0 - l1 * bx.e2;
   const int lo1 = wrap_near(bx.lo[0], d.n1), lo2 = wrap_near(bx.lo[1], d.n2);
-  unsigned dst = (unsigned)__cvta_generic_to_shared(sb) + 4u * (unsigned)(r0 * kPitch + 4 * lc);  // Q = e2 P
+  unsigned dst = (unsigned)__cvta_generic_to_shared(sb) + 4u * (unsigned)(r0 * bx.P + 4 * lc);  // Q = e2 P
   while (l1 < bx.e1) {
     int g1 = lo1 + l1, g2 = lo2 + l2;
     g1 -= g1 >= d.n1 ? d.n1 : 0;
@@ -316,7 +321,7 @@ CB_DEVICE void issue_box(float* sb, const float* __restrict__ f, const TileBox& 
     const float* src = f + (unsigned)(g1 * d.n2 + g2) * (unsigned)d.n3;
     copy16(dst, src + g3);
     if (hi) copy16(dst + 128u, src + h3);
-    dst += 4u * kRows * kPitch;
+    dst += 4u * kRows * (unsigned)bx.P;
     l1 += s1;
     l2 += s2;
     if (l2 >= bx.e2) {
@@ -351,14 +356,14 @@ CB_DEVICE void issue_box(float* __restrict__ sb, const bf16* __restrict__ f, con
   constexpr int kWarps = kTileThreads / 32;
   for (int l1 = warp; l1 < bx.e1; l1 += kWarps) {
     const bf16* fp = fb + (unsigned)g1 * plane;
-    float* sp = sb + l1 * bx.Q + lr * kPitch + 4 * lc;
+    float* sp = sb + l1 * bx.Q + lr * bx.P + 4 * lc;
     int g2 = w2;
     for (int l2 = lr; l2 < bx.e2; l2 += rpi) {
       const uint2 raw = __ldg(reinterpret_cast<const uint2*>(fp + (unsigned)g2 * row));
       const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
       const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
       *reinterpret_cast<float4*>(sp) = make_float4(lo.x, lo.y, hi.x, hi.y);
-      sp += rpi * kPitch;
+      sp += rpi * bx.P;
       g2 += rpi;
       while (g2 >= d.n2) g2 -= d.n2;
     }
@@ -451,11 +456,11 @@ CB_DEVICE void row1(unsigned addr, float (&x)[NC]) {
   x[3] = lds<OFF + 12>(addr);
   if constexpr (NC > 4) x[4] = lds<OFF + 16>(addr);
 }
-template <int OFF, int NC>
+template <int OFF, int P, int NC>
 CB_DEVICE void rows2(unsigned addr, f32x2 (&x)[NC]) {
   float a[NC], b[NC];
   row1<OFF>(addr, a);
-  row1<OFF + 8 * kPitch>(addr, b);
+  row1<OFF + 8 * P>(addr, b);
 #pragma unroll
   for (int c = 0; c < NC; ++c) x[c] = pk2(a[c], b[c]);
 }
@@ -505,6 +510,7 @@ struct PairWeights {
 // Points A (planes 0..3 from base) and B (planes 1..4) in one pass over five
 // planes qb bytes apart; `last` is the address of plane 4 (any box address where
 // B is not wanted).  One row pair is live at a time.
+template <int P>
 CB_DEVICE float2 gather_pair(unsigned base, unsigned qb, unsigned last, const PairWeights& w) {
   float ra = 0.f, rb = 0.f;
 #pragma unroll
@@ -513,13 +519,13 @@ CB_DEVICE float2 gather_pair(unsigned base, unsigned qb, unsigned last, const Pa
     f32x2 ta = 0ull, tb = 0ull;
     {
       f32x2 x[4];
-      rows2<0>(pa, x);
+      rows2<0, P>(pa, x);
       if (q < 4) ta = mul2(w.w2[0][0], row_sums(x, w.w3[0]));
       if (q > 0) tb = mul2(w.w2[1][0], row_sums(x, w.w3[1]));
     }
     {
       f32x2 x[4];
-      rows2<4 * kPitch>(pa, x);
+      rows2<4 * P, P>(pa, x);
       if (q < 4) ta = fma2(w.w2[0][1], row_sums(x, w.w3[0]), ta);
       if (q > 0) tb = fma2(w.w2[1][1], row_sums(x, w.w3[1]), tb);
     }
@@ -538,18 +544,19 @@ CB_DEVICE float2 gather_pair(unsigned base, unsigned qb, unsigned last, const Pa
 // Fractions s of displacement dd and the shared address of the stencil's first
 // tap, `origin` being the address of the tap at floor(d) = 0.  Addresses
 // o1 Q + o2 P + o3 (o2 < ext2, o3 < P) are distinct for distinct taps.
+template <int P>
 CB_DEVICE unsigned point_stencil(const float (&dd)[3], unsigned origin, unsigned qb, float (&s)[3]) {
   const float f1 = floorf(dd[0]), f2 = floorf(dd[1]), f3 = floorf(dd[2]);
   s[0] = dd[0] - f1;
   s[1] = dd[1] - f2;
   s[2] = dd[2] - f3;
-  return origin + (unsigned)(int)f1 * qb + (unsigned)(int)f2 * (4 * kPitch) + 4u * (unsigned)(int)f3;
+  return origin + (unsigned)(int)f1 * qb + (unsigned)(int)f2 * (4 * P) + 4u * (unsigned)(int)f3;
 }
 
 // Address of the first tap of point (x1, x2, x3) at floor(d) = 0 (taken modulo
 // 2^32: it may lie outside the box).
 CB_DEVICE unsigned tap_origin(unsigned sb, int x1, int x2, int x3, const TileBox& bx) {
-  return sb + 4u * (unsigned)((x1 - 1 - bx.lo[0]) * bx.Q + (x2 - 1 - bx.lo[1]) * kPitch + (x3 - 1 - bx.lo[2]));
+  return sb + 4u * (unsigned)((x1 - 1 - bx.lo[0]) * bx.Q + (x2 - 1 - bx.lo[1]) * bx.P + (x3 - 1 - bx.lo[2]));
 }
 
 // Points of the tile that are gathered one by one.
@@ -569,7 +576,7 @@ struct PointList {
 
 // Staged gather of the tile's points: epi(index, value, aux) for every point
 // inside the grid.  Contains __syncthreads: call from uniform control flow.
-template <class Src, class Epi>
+template <int P, class Src, class Epi>
 CB_DEVICE void gather_tile(unsigned sb, const PointList& list, const Src& src, const float (&dd)[kTilePts][3],
                            const float (&aux)[kTilePts], const TileThread& tt, const TileBox& bx, const Dims& d,
                            const TileGrid& tg, const Epi& epi) {
@@ -578,11 +585,11 @@ CB_DEVICE void gather_tile(unsigned sb, const PointList& list, const Src& src, c
 #pragma unroll
   for (int a = 0; a < kTilePts; a += 2) {
     float s[3], t[3];
-    const unsigned base = point_stencil(dd[a], origin + (unsigned)tt.step(a) * qb, qb, s);
-    const unsigned baseb = point_stencil(dd[a + 1], origin + (unsigned)tt.step(a + 1) * qb, qb, t);
+    const unsigned base = point_stencil<P>(dd[a], origin + (unsigned)tt.step(a) * qb, qb, s);
+    const unsigned baseb = point_stencil<P>(dd[a + 1], origin + (unsigned)tt.step(a + 1) * qb, qb, t);
     const bool shared = baseb == base + qb;
     list.push(tt.valid(a + 1) && !shared, a + 1);
-    const float2 r = gather_pair(base, qb, shared ? base + 4 * qb : base, PairWeights(s, t));
+    const float2 r = gather_pair<P>(base, qb, shared ? base + 4 * qb : base, PairWeights(s, t));
     if (tt.valid(a)) epi(tt.idx(a), r.x, aux[a]);
     if (shared && tt.valid(a + 1)) epi(tt.idx(a + 1), r.y, aux[a + 1]);
   }
@@ -600,11 +607,37 @@ CB_DEVICE void gather_tile(unsigned sb, const PointList& list, const Src& src, c
     float de[3], s[3], w1[4], w2[4], w3[4];
     src.at(de, at, d);
     const float ae = epi.aux ? __ldg(epi.aux + at) : 0.f;
-    const unsigned base = point_stencil(de, tap_origin(sb, x1, x2, x3, bx), qb, s);
+    const unsigned base = point_stencil<P>(de, tap_origin(sb, x1, x2, x3, bx), qb, s);
     lagrange4(s[0], w1);
     lagrange4(s[1], w2);
     lagrange4(s[2], w3);
-    epi(at, gather_box<kPitch>(base, qb, w1, w2, w3), ae);
+    epi(at, gather_box<P>(base, qb, w1, w2, w3), ae);
+  }
+}
+
+// The same for the few tiles whose box is only staged at the tight pitch: point
+// by point, plane by plane, in few registers (a second copy of the pair pass
+// makes the common one spill).
+template <class Epi>
+CB_DEVICE void gather_tight(unsigned sb, const float (&dd)[kTilePts][3], const float (&aux)[kTilePts],
+                            const TileThread& tt, const TileBox& bx, const Epi& epi) {
+  const unsigned qb = (unsigned)bx.Q * 4u;
+  const unsigned origin = tap_origin(sb, tt.x1_, tt.x2, tt.x3, bx);
+#pragma unroll
+  for (int a = 0; a < kTilePts; ++a) {
+    float s[3], w1[4], w2[4], w3[4];
+    unsigned at = point_stencil<kPitchTight>(dd[a], origin + (unsigned)tt.step(a) * qb, qb, s);
+    lagrange4(s[0], w1);
+    lagrange4(s[1], w2);
+    lagrange4(s[2], w3);
+    float r = 0.f;
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q, at += qb) {
+      const float w = q < 2 ? (q ? w1[1] : w1[0]) : (q == 2 ? w1[2] : w1[3]);
+      r += w * (w2[0] * row4<0>(at, w3) + w2[1] * row4<4 * kPitchTight>(at, w3) +
+                w2[2] * row4<8 * kPitchTight>(at, w3) + w2[3] * row4<12 * kPitchTight>(at, w3));
+    }
+    if (tt.valid(a)) epi(tt.idx(a), r, aux[a]);
   }
 }
 
@@ -698,7 +731,9 @@ CB_DEVICE void tile_gather(float* sb, const Src& src, const int4* __restrict__ t
     // registers (here, after every load is issued: the statement waits for dd)
 #pragma unroll
     for (int a = 0; a < kTilePts; ++a) asm volatile("" : "+f"(dd[a][0]), "+f"(dd[a][1]), "+f"(dd[a][2]));
-    gather_tile(sbase, point_list(sb, &listed[k & 1]), src, dd, aux, tt, bx, d, tg, e);
+    const PointList list = point_list(sb, &listed[k & 1]);
+    if (bx.P == kPitch) gather_tile<kPitch>(sbase, list, src, dd, aux, tt, bx, d, tg, e);
+    else gather_tight(sbase, dd, aux, tt, bx, e);
   }
 }
 
@@ -720,7 +755,10 @@ CB_DEVICE void tile_step(float* sb, const Src& src, const int4* __restrict__ tab
   if (!staged) return gather_unstaged(f, dd, aux, tt, d, e);
   copies_landed();
   __syncthreads();
-  gather_tile((unsigned)__cvta_generic_to_shared(sb), point_list(sb, &listed), src, dd, aux, tt, bx, d, tg, e);
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(sb);
+  const PointList list = point_list(sb, &listed);
+  if (bx.P == kPitch) gather_tile<kPitch>(sbase, list, src, dd, aux, tt, bx, d, tg, e);
+  else gather_tight(sbase, dd, aux, tt, bx, e);
 }
 
 }  // namespace cb

@@ -44,7 +44,9 @@ def smooth(rng, shape, amp, kmax=3):
 # (shape, largest displacement in cells): whole and partial tiles, floors that
 # change inside a pair, boxes up to and beyond the staging limit
 CASES = [((16, 16, 32), 0.4), ((17, 23, 36), 0.9), ((33, 9, 20), 1.7), ((40, 24, 52), 3.0), ((24, 40, 64), 9.0),
-         ((21, 19, 30), 1.0), ((96, 80, 96), 2.5), ((97, 70, 100), 1.3)]
+         ((21, 19, 30), 1.0), ((96, 80, 96), 2.5), ((97, 70, 100), 1.3),
+         # strong maps: boxes that are staged only at the tight row pitch
+         ((64, 64, 64), 6.0), ((72, 56, 96), 7.0)]
 
 
 @pytest.mark.parametrize("shape,amp", CASES)
