@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
   extern __shared__ __align__(16) float sbuf[];
   float* o = out + p * op + k0 * of;
   tile_gather(sbuf, DispSource{disp + p * dp}, tab ? tab + p * tp : nullptr, f + p * fp + k0 * ff, ff,
-                     min(nfz, nf - k0), d, tg, [&](int i) { return StoreEpi{o + i * of, nullptr}; });
+              min(nfz, nf - k0), d, tg, [&](int i) { return StoreEpi{o + i * of, nullptr}; });
 }
 
 // one bf16 field without a box table
@@ -218,7 +218,8 @@ __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
 __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
     k_gather_add(const float* __restrict__ f, long long fp, const float* __restrict__ disp, long long dp,
                  const int4* __restrict__ tab, long long tp, const float* __restrict__ s, long long sp,
-                 float* __restrict__ out, long long op, float sign, Dims d, TileGrid tg, const int* __restrict__ active) {
+                 float* __restrict__ out, long long op, float sign, Dims d, TileGrid tg,
+                 const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
   extern __shared__ __align__(16) float sbuf[];
@@ -239,8 +240,8 @@ __global__ void __launch_bounds__(kTileThreads, kGatherMinBlocks)
 
 // Box table of a displacement field (sl_tile.cuh box_from_table layout).
 __global__ void __launch_bounds__(kTileThreads)
-    k_tile_table(const float* __restrict__ disp, long long dp, int4* __restrict__ tab, long long tp, Dims d, TileGrid tg,
-                 const int* __restrict__ active) {
+    k_tile_table(const float* __restrict__ disp, long long dp, int4* __restrict__ tab, long long tp, Dims d,
+                 TileGrid tg, const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (active && !active[p]) return;
   const TileThread tt = tile_thread(d, tg);
@@ -410,12 +411,6 @@ int launch_interp(const float* f, long long fp, long long ff, const float* disp,
   return (int)cudaGetLastError();
 }
 
-// Whether one gather at a new displacement should build its table first: the
-// table's own pass costs less than the reduction inside each gather CTA once the
-// tiles fill the GPU (256^3: 37 + 179 us against 217; 128^3: 6 + 27 against 32);
-// below that it is one more launch (64^3: 2.4 + 7.5 against 8.1).
-bool interp_wants_table(const Dims& d) { return tile_count(d) >= 4 * 148; }
-
 int launch_interp16(const bf16* f, long long fp, const float* disp, long long dp, const int4* tab, long long tp,
                     bf16* out, long long op, int nprob, const Dims& d, const int* active, cudaStream_t s) {
   // staged boxes load 4-element chunks as 8-byte words (only when N3 % 4 == 0)
@@ -428,8 +423,8 @@ int launch_interp16(const bf16* f, long long fp, const float* disp, long long dp
   }
   int e = allow_smem(k_interp16);
   if (e) return e;
-  k_interp16<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(f, fp, disp, dp, tab, tp, out, op, d, TileGrid(d),
-                                                                            active);
+  k_interp16<<<tile_grid(d, nprob, 1), kTileThreads, kGatherSmemBytes, s>>>(f, fp, disp, dp, tab, tp, out, op, d,
+                                                                            TileGrid(d), active);
   return (int)cudaGetLastError();
 }
 

@@ -97,9 +97,6 @@ int launch_tile_table(const float* disp, long long dp, int4* tab, long long tp, 
                       const int* active, cudaStream_t s);
 long long tile_table_int4s(const Dims& d);
 
-// Whether a single gather at a displacement should build its table first.
-bool interp_wants_table(const Dims& d);
-
 // out[p][f] <- f[p][f](i + disp[p](i)), f = 0..nf-1; fields ff apart; tab =
 // disp's box table (null: every CTA reduces its box itself).
 int launch_interp(const float* f, long long fp, long long ff, const float* disp, long long dp, const int4* tab,

@@ -1,9 +1,8 @@
 """Tile gathers where their paths meet: tiles that stick out of the grid (odd
 lengths), pairs of points whose stencils differ, boxes that are too large or
 too wide to stage, rows that cannot be copied in 16-byte chunks, fields that
-start off a 16-byte boundary, one and three fields, with and without a box
-table (launches below and above one wave of tiles), and values that are not
-finite."""
+start off a 16-byte boundary, one and three fields, launches below and above
+one wave of tiles, and values that are not finite."""
 import numpy as np
 import pytest
 
