@@ -16,9 +16,8 @@
 // the 1D transform along axis k, so gradient and divergence are one pass per
 // axis over real data.
 //
-// Every global->shared load is two-phase: a thread issues all of its loads
-// into registers (compile-time count) before it stores any of them, so each
-// thread keeps 8-32 independent loads in flight.
+// A butterfly's elements go straight between global memory and registers (a
+// compile-time count of independent loads per thread, 4-32 in flight).
 #include <atomic>
 #include <cstdio>
 #include <mutex>
@@ -126,8 +125,9 @@ CB_DEVICE bool epi_reduces(int epi) { return epi == EPI_SUMSQ || epi == EPI_STOR
 template <class F>
 CB_DEVICE void rows_a(const float* __restrict__ ra, bool ok, int p, int j, float2* S) {
   const float* rb = ra + F::R0 * F::R1;
-  fft_a<F::R0, F::R1, false>(j, [&](int e) { return ok ? make_float2(__ldg(ra + e), __ldg(rb + e)) : make_float2(0.f, 0.f); },
-                             [&](int k0, float2 v) { S[p * F::PL + k0 * F::PK + j] = v; });
+  fft_a<F::R0, F::R1, false>(
+      j, [&](int e) { return ok ? make_float2(__ldg(ra + e), __ldg(rb + e)) : make_float2(0.f, 0.f); },
+      [&](int k0, float2 v) { S[p * F::PL + k0 * F::PK + j] = v; });
 }
 
 // Inverse A butterfly and the epilogue: value e of row a / b is al times the
@@ -301,7 +301,8 @@ __global__ void __launch_bounds__(RowCfg<N, V>::T, 1024 / RowCfg<N, V>::T)
 // column g starts at (g / cpg) * gs + (g % cpg); elements are es apart
 // ---------------------------------------------------------------------------
 template <int N, bool INV, int V>
-__global__ void __launch_bounds__(ColCfg<N, V>::T, 1024 / ColCfg<N, V>::T) k_cols(float2* __restrict__ data, long long pstr, long long fstr,
+__global__ void __launch_bounds__(ColCfg<N, V>::T, 1024 / ColCfg<N, V>::T)
+    k_cols(float2* __restrict__ data, long long pstr, long long fstr,
                                                            int ncols, int cpg, long long gs, int es,
                                                            const float2* __restrict__ twg,
                                                            const int* __restrict__ active) {
@@ -497,7 +498,8 @@ struct DiagSymbol {
 // passes through shared memory and the symbol per field (traffic floor 62 us);
 // 128^3: 16 against 22.
 template <int N, int V, bool DIAG>
-__global__ void __launch_bounds__(ColCfg<N, V>::T, (DIAG ? (ColCfg<N, V>::R1 > 12 ? 768 : 1024) : 512) / ColCfg<N, V>::T)
+__global__ void __launch_bounds__(ColCfg<N, V>::T,
+                                  (DIAG ? (ColCfg<N, V>::R1 > 12 ? 768 : 1024) : 512) / ColCfg<N, V>::T)
     k_pencil1(float2* __restrict__ spec, long long pstr, long long fstr, int nf, Dims d, int op, float s,
               const SpecParams* __restrict__ params, SpecParams one, const float2* __restrict__ twg,
               const int* __restrict__ active) {
@@ -567,7 +569,8 @@ __global__ void __launch_bounds__(ColCfg<N, V>::T, (DIAG ? (ColCfg<N, V>::R1 > 1
 // spectra of an element meet in one thread's registers (128^3: 14 us, 24 when
 // they were staged in shared memory between the transforms).
 template <int N, int V>
-__global__ void __launch_bounds__(ColCfg<N, V>::T, 512 / ColCfg<N, V>::T) k_pencil3(float2* __restrict__ spec, long long pstr,
+__global__ void __launch_bounds__(ColCfg<N, V>::T, 512 / ColCfg<N, V>::T)
+    k_pencil3(float2* __restrict__ spec, long long pstr,
                                                               long long fstr, Dims d, int op, float s,
                                                               const SpecParams* __restrict__ params,
                                                               SpecParams one, const float2* __restrict__ twg,
@@ -676,7 +679,8 @@ __global__ void __launch_bounds__(RowCfg<N, V>::T, 1024 / RowCfg<N, V>::T)
 // between the forward and the inverse B butterfly.  One 128^3 field: 7.4 us,
 // 9.1 with 4-byte accesses and four staged passes.
 template <int N, int V>
-__global__ void __launch_bounds__(ColCfg<N, V>::T, 1024 / ColCfg<N, V>::T) k_deriv_cols(const float* __restrict__ in, long long ip,
+__global__ void __launch_bounds__(ColCfg<N, V>::T, 1024 / ColCfg<N, V>::T)
+    k_deriv_cols(const float* __restrict__ in, long long ip,
                                                                  long long ifs, float* __restrict__ out,
                                                                  long long op, long long ofs, int ncols, int cpg,
                                                                  long long gs, int es,
