@@ -792,7 +792,7 @@ int claire_b200_trajectory(const float* v, float* disp, const int nx[3], int nt,
 // A gather at a displacement used once builds no table: its CTAs reduce their
 // boxes themselves (the reduction overlaps other CTAs' gathers, a table is one
 // more pass over the displacement and one more launch).  Table + gather against
-// one kernel: 128^3 37.0 / 32.8 us, 256^3 219 / 214, three fields of 256^3
+// one kernel: 128^3 37.0 / 31.1 us, 256^3 219 / 202, three fields of 256^3
 // 539 / 515, bf16 256^3 245 / 231; faster at every size from 96^3.
 int claire_b200_interp3(const float* f, const float* disp, float* out, const int nx[3], int dof, void* stream) {
   if (!f || !disp || !out || !dims_ok(nx) || (dof != 1 && dof != 3)) return CB_ERR_ARG;

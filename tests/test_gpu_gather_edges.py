@@ -61,6 +61,16 @@ def test_interpolation(cb, shape, amp):
     assert rel(one, ref[1]) < TOL
 
 
+@pytest.mark.parametrize("shape,amp", CASES)
+def test_one_field(cb, shape, amp):
+    rng = np.random.default_rng(sum(shape) + 1)
+    disp = smooth(rng, shape, amp)
+    f = rng.standard_normal(shape).astype(np.float32)
+    ref = R.interp3(f.astype(np.float64), R.index_grid(shape) + disp.astype(np.float64))
+    out = cb.SemiLagrangian.Interpolate(to_dev(f), to_dev(disp)).cpu().numpy()
+    assert rel(out, ref) < TOL
+
+
 @pytest.mark.parametrize("shape,amp", [((16, 16, 32), 0.4), ((40, 24, 52), 3.0), ((97, 70, 100), 1.3)])
 def test_field_off_a_16_byte_boundary(cb, shape, amp):
     import torch
