@@ -922,13 +922,14 @@ static int spectral3(const float* in, float* out, const Dims& d, int op, const S
                      double* sumsq, cudaStream_t st) {
   Scratch sc;
   const int np = epi == EPI_SUMSQ ? std::max(1, c2r_partials(d, 3)) : 0;
+  int used = 0;
   int e = sc.alloc(d, 3, np, st);
   if (e) return e;
   const long long n = d.n(), nc = d.nc();
   e = launch_r2c3d(in, 0, n, sc.spec, 0, 3, 1, d, nullptr, st);
   if (!e) e = launch_pencil(sc.spec, 0, 1, d, op, nullptr, 3, 3, nullptr, st, &hp);
-  if (!e) e = launch_c2r3d(sc.spec, 0, out, 0, n, 3, 1, d, epi, nullptr, sc.partials, np, nullptr, st);
-  if (!e && epi == EPI_SUMSQ) e = launch_finalize(sc.partials, np, np, sc.result, 1, 1.0, false, st);
+  if (!e) e = launch_c2r3d(sc.spec, 0, out, 0, n, 3, 1, d, epi, nullptr, sc.partials, np, nullptr, st, nullptr, &used);
+  if (!e && epi == EPI_SUMSQ) e = launch_finalize(sc.partials, np, used, sc.result, 1, 1.0, false, st);
   note_launches(6);
   if (e) return cuda_status(e);
   if (epi == EPI_SUMSQ && sumsq) {
@@ -978,8 +979,8 @@ int claire_b200_reg_functional(const float* v, double* R, const int nx[3], int r
     int e = 0;
     if (regnorm != CB_NORM_L2) {
       for (int a = 0; a < 3 && !e; ++a) {
-        const int p = deriv_partials(d, a, 3);
-        e = launch_deriv(v, 0, n, nullptr, 0, 0, 3, 1, d, a, EPI_SUMSQ, buf, np, nullptr, st);
+        int p = 0;
+        e = launch_deriv(v, 0, n, nullptr, 0, 0, 3, 1, d, a, EPI_SUMSQ, buf, np, nullptr, st, &p);
         if (!e) e = launch_finalize(buf, np, p, res, 1, 1.0, a > 0, st);
       }
       note_launches(6);

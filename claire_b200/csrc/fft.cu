@@ -114,7 +114,9 @@ template <int N, int V = 0> struct ColCfg {
   static_assert(T % C == 0, "a thread keeps its column");
 };
 
-CB_DEVICE bool epi_reduces(int epi) { return epi == EPI_SUMSQ || epi == EPI_STORE_DOT || epi == EPI_ADD_DOT; }
+__host__ __device__ inline bool epi_reduces(int epi) {
+  return epi == EPI_SUMSQ || epi == EPI_STORE_DOT || epi == EPI_ADD_DOT;
+}
 
 // ---------------------------------------------------------------------------
 // rows (x3).  Two real rows a, b (2p and 2p + 1) are packed as z = a + i b.
@@ -852,7 +854,8 @@ int set_fft_variant(int n, int v) {
     switch (fft_variant(N_)) { CB_V(0, CALL) CB_V(1, CALL)                                 \
       default: return (int)cudaErrorInvalidValue; }                                        \
   } break;
-// CB_DISPATCH_N with the size's current variant as the constexpr VV
+// CB_DISPATCH_N with the size's current variant as the constexpr VV.  It is read
+// once: kernel, grid and the count of partials of a launch belong together.
 #define CB_DISPATCH_NV(n, CALL)      \
   switch (n) {                       \
     case 16: CB_VSW2(16, CALL)       \
@@ -880,6 +883,15 @@ int set_fft_variant(int n, int v) {
     default: return (int)cudaErrorInvalidValue; \
   }
 
+// Partials of a reducing launch: reported through *used; an error where they do
+// not fit into nparts.
+static int claim_partials(int epi, const dim3& grid, const double* partials, int nparts, int* used) {
+  const int count = (int)(grid.x * grid.y);
+  if (used) *used = epi_reduces(epi) ? count : 0;
+  if (epi_reduces(epi) && (!partials || !used || count > nparts)) return (int)cudaErrorInvalidValue;
+  return 0;
+}
+
 template <int N, int V>
 static int r2c_rows_impl(const float* in, long long ip, long long ifs, float2* out, long long op,
                          long long ofs, int nrows, int nf, int nprob, const int* active,
@@ -897,13 +909,15 @@ static int r2c_rows_impl(const float* in, long long ip, long long ifs, float2* o
 template <int N, int V>
 static int c2r_rows_impl(const float2* in, long long ip, long long ifs, float* out, long long op,
                          long long ofs, int nrows, int nf, int nprob, int epi, const float* alpha,
-                         double* partials, int nparts, const float* other, const int* active, cudaStream_t s) {
+                         double* partials, int nparts, int* used, const float* other, const int* active,
+                         cudaStream_t s) {
   const float2* tw = twiddles(N);
   if (!tw) return (int)cudaErrorMemoryAllocation;
   size_t sm = RowCfg<N, V>::smem;
-  int e = set_smem(k_c2r_rows<N, V>, sm);
-  if (e) return e;
   dim3 grid((nrows + 2 * RowCfg<N, V>::P - 1) / (2 * RowCfg<N, V>::P), nf, nprob);
+  int e = claim_partials(epi, grid, partials, nparts, used);
+  if (!e) e = set_smem(k_c2r_rows<N, V>, sm);
+  if (e) return e;
   k_c2r_rows<N, V><<<grid, RowCfg<N, V>::T, sm, s>>>(in, ip, ifs, out, op, ofs, nrows, tw, epi, alpha, partials,
                                             nparts, other, active);
   return (int)cudaGetLastError();
@@ -985,9 +999,9 @@ int launch_pencil(float2* spec, long long sp, int nprob, const Dims& d, int op,
   return e;
 }
 
-// Lines per CTA of the size's current variant (min_over_variants: the
-// smallest over its candidates, which sizes reduction buffers for any variant).
-static int row_lines(int n, bool min_over_variants = false) {
+// Packed lines per CTA: the smallest over the size's variants, which sizes
+// reduction buffers for any of them.
+static int row_lines(int n) {
   auto pairs = [](int k, int v) {
     switch (k) {
       case 16: return row_pairs((v & 1) ? RowPlan<16, 1>::R1 : RowPlan<16, 0>::R1, v);
@@ -1001,13 +1015,12 @@ static int row_lines(int n, bool min_over_variants = false) {
       default: return 0;
     }
   };
-  if (!min_over_variants) return pairs(n, fft_variant(n));
   int m = pairs(n, 0);
   for (int v = 1; v < 4; ++v) m = pairs(n, v) < m ? pairs(n, v) : m;
   return m;
 }
 
-static int col_lines(int n, bool min_over_variants = false) {
+static int col_lines(int n) {
   int base = 0, alt = 0;
   switch (n) {
     case 16: base = ColLines<16>::base; alt = ColLines<16>::alt; break;
@@ -1021,12 +1034,11 @@ static int col_lines(int n, bool min_over_variants = false) {
     case 150: base = ColLines<150>::base; alt = ColLines<150>::alt; break;
     default: return 0;
   }
-  if (min_over_variants) return base < alt ? base : alt;
-  return (fft_variant(n) & 2) ? alt : base;
+  return base < alt ? base : alt;
 }
 
-int c2r_partials(const Dims& d, int nf, bool any_variant) {
-  const int P = row_lines(d.n3, any_variant);
+int c2r_partials(const Dims& d, int nf) {
+  const int P = row_lines(d.n3);
   if (!P) return 0;
   const int nrows = d.n1 * d.n2;
   return ((nrows + 2 * P - 1) / (2 * P)) * nf;
@@ -1034,7 +1046,7 @@ int c2r_partials(const Dims& d, int nf, bool any_variant) {
 
 int launch_c2r3d(float2* spec, long long sp, float* out, long long op_, long long ofs, int nf,
                  int nprob, const Dims& d, int epi, const float* alpha, double* partials, int nparts,
-                 const int* active, cudaStream_t s, const float* other) {
+                 const int* active, cudaStream_t s, const float* other, int* used) {
   if ((epi == EPI_STORE_DOT || epi == EPI_ADD_DOT || epi == EPI_SUM) && !other) return (int)cudaErrorInvalidValue;
   if (!axes_supported(d)) return (int)cudaErrorInvalidValue;
   const long long nc = d.nc();
@@ -1044,21 +1056,22 @@ int launch_c2r3d(float2* spec, long long sp, float* out, long long op_, long lon
                                                nf, nprob, active, s)));
   if (e) return e;
   CB_DISPATCH_NV(d.n3, e = (c2r_rows_impl<NN, VV>(spec, sp, nc, out, op_, ofs, d.n1 * d.n2, nf, nprob, epi, alpha,
-                                            partials, nparts, other, active, s)));
+                                            partials, nparts, used, other, active, s)));
   return e;
 }
 
 template <int N, int V>
 static int deriv_rows_impl(const float* in, long long ip, long long ifs, float* out, long long op_, long long ofs,
-                           int nf, int nprob, const Dims& d, int epi, double* partials, int nparts,
+                           int nf, int nprob, const Dims& d, int epi, double* partials, int nparts, int* used,
                            const int* active, cudaStream_t s) {
   const float2* tw = twiddles(N);
   if (!tw) return (int)cudaErrorMemoryAllocation;
   size_t sm = RowCfg<N, V>::smem;
-  int e = set_smem(k_deriv_rows<N, V>, sm);
-  if (e) return e;
   const int nrows = d.n1 * d.n2;
   dim3 grid((nrows + 2 * RowCfg<N, V>::P - 1) / (2 * RowCfg<N, V>::P), nf, nprob);
+  int e = claim_partials(epi, grid, partials, nparts, used);
+  if (!e) e = set_smem(k_deriv_rows<N, V>, sm);
+  if (e) return e;
   k_deriv_rows<N, V><<<grid, RowCfg<N, V>::T, sm, s>>>(in, ip, ifs, out, op_, ofs, nrows, tw, epi, partials, nparts, active);
   return (int)cudaGetLastError();
 }
@@ -1066,12 +1079,10 @@ static int deriv_rows_impl(const float* in, long long ip, long long ifs, float* 
 template <int N, int V>
 static int deriv_cols_impl(const float* in, long long ip, long long ifs, float* out, long long op_, long long ofs,
                            int nf, int nprob, const Dims& d, int axis, int epi, double* partials, int nparts,
-                           const int* active, cudaStream_t s) {
+                           int* used, const int* active, cudaStream_t s) {
   const float2* tw = twiddles(N);
   if (!tw) return (int)cudaErrorMemoryAllocation;
   size_t sm = col_smem<N, V>(1);
-  int e = set_smem(k_deriv_cols<N, V>, sm);
-  if (e) return e;
   // neighbouring columns as one float2: even strides and 8-byte bases
   auto pairs = [](const float* p, long long a, long long b) {
     return (reinterpret_cast<uintptr_t>(p) & 7) == 0 && ((a | b) & 1) == 0;
@@ -1085,20 +1096,23 @@ static int deriv_cols_impl(const float* in, long long ip, long long ifs, float* 
   }
   constexpr int C = 2 * ColCfg<N, V>::C;
   dim3 grid((ncols + C - 1) / C, nf, nprob);
+  int e = claim_partials(epi, grid, partials, nparts, used);
+  if (!e) e = set_smem(k_deriv_cols<N, V>, sm);
+  if (e) return e;
   k_deriv_cols<N, V><<<grid, ColCfg<N, V>::T, sm, s>>>(in, ip, ifs, out, op_, ofs, ncols, cpg, gs, (int)es, tw, epi,
                                                        pairs(in, ip, ifs), pairs(out, op_, ofs), partials, nparts,
                                                        active);
   return (int)cudaGetLastError();
 }
 
-int deriv_partials(const Dims& d, int axis, int nf, bool any_variant) {
+int deriv_partials(const Dims& d, int axis, int nf) {
   const int n = (axis == 0) ? d.n1 : (axis == 1 ? d.n2 : d.n3);
   if (axis == 2) {
-    const int P = row_lines(n, any_variant);
+    const int P = row_lines(n);
     if (!P) return 0;
     return ((d.n1 * d.n2 + 2 * P - 1) / (2 * P)) * nf;
   }
-  const int C = col_lines(n, any_variant);
+  const int C = col_lines(n);
   if (!C) return 0;
   const int ncols = (axis == 1) ? d.n1 * d.n3 : d.n2 * d.n3;
   return ((ncols + 2 * C - 1) / (2 * C)) * nf;
@@ -1106,17 +1120,17 @@ int deriv_partials(const Dims& d, int axis, int nf, bool any_variant) {
 
 int launch_deriv(const float* in, long long ip, long long ifs, float* out, long long op_,
                  long long ofs, int nf, int nprob, const Dims& d, int axis, int epi,
-                 double* partials, int nparts, const int* active, cudaStream_t s) {
+                 double* partials, int nparts, const int* active, cudaStream_t s, int* used) {
   if (!axes_supported(d)) return (int)cudaErrorInvalidValue;
   if (axis == 2 && (!aligned16(in) || ((ip | ifs) & 3))) return (int)cudaErrorInvalidValue;
   const int n = (axis == 0) ? d.n1 : (axis == 1 ? d.n2 : d.n3);
   int e = 0;
   if (axis == 2) {
     CB_DISPATCH_NV(n, e = (deriv_rows_impl<NN, VV>(in, ip, ifs, out, op_, ofs, nf, nprob, d, epi, partials, nparts,
-                                                   active, s)));
+                                                   used, active, s)));
   } else {
     CB_DISPATCH_NV_COL(n, e = (deriv_cols_impl<NN, VV>(in, ip, ifs, out, op_, ofs, nf, nprob, d, axis, epi,
-                                                       partials, nparts, active, s)));
+                                                       partials, nparts, used, active, s)));
   }
   return e;
 }

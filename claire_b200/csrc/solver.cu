@@ -163,8 +163,8 @@ int Solver::alloc(void** p, size_t bytes) {
 
 static int max_parts(const Dims& d) {
   int mp = dot_partials(3 * d.n());
-  for (int a = 0; a < 3; ++a) mp = std::max(mp, deriv_partials(d, a, 3, true));
-  mp = std::max(mp, c2r_partials(d, 3, true));
+  for (int a = 0; a < 3; ++a) mp = std::max(mp, deriv_partials(d, a, 3));
+  mp = std::max(mp, c2r_partials(d, 3));
   mp = std::max(mp, 3 * field_stats_parts(d.n()));
   return mp;
 }
@@ -711,8 +711,8 @@ int Solver::reg_functional(const float* vel, const std::vector<int>& sel, const 
     // sum_i sum_k ||d/dx_k v_i||^2 with spectral derivatives (src/RegularizationH1SN.cpp:84-141)
     CB_TRY(upload_mask(ma, dma));
     for (int a = 0; a < 3; ++a) {
-      const int np = deriv_partials(d, a, 3);
-      CB_TRY(launch_deriv(vel, 3 * n, n, nullptr, 0, 0, 3, B, d, a, EPI_SUMSQ, partials, maxparts, dma, stream));
+      int np = 0;
+      CB_TRY(launch_deriv(vel, 3 * n, n, nullptr, 0, 0, 3, B, d, a, EPI_SUMSQ, partials, maxparts, dma, stream, &np));
       CB_TRY(launch_finalize(partials, maxparts, np, slot(S_R), B, 1.0, a > 0, stream, dma));
     }
     note_launches(6);
@@ -722,8 +722,9 @@ int Solver::reg_functional(const float* vel, const std::vector<int>& sel, const 
     CB_TRY(upload_mask(mb, dmb));
     CB_TRY(launch_r2c3d(vel, 3 * n, n, spec, 3 * nc, 3, B, d, dmb, stream));
     CB_TRY(launch_pencil(spec, 3 * nc, B, d, OP_REG_FUNC, dparams, 3, 3, dmb, stream));
-    const int np = c2r_partials(d, 3);
-    CB_TRY(launch_c2r3d(spec, 3 * nc, nullptr, 0, 0, 3, B, d, EPI_SUMSQ, nullptr, partials, maxparts, dmb, stream));
+    int np = 0;
+    CB_TRY(launch_c2r3d(spec, 3 * nc, nullptr, 0, 0, 3, B, d, EPI_SUMSQ, nullptr, partials, maxparts, dmb, stream,
+                        nullptr, &np));
     // finalize only the selected problems' slots: unselected keep stale values
     CB_TRY(launch_finalize(partials, maxparts, np, slot(S_R), B, 1.0, false, stream, dmb));
     note_launches(6);
@@ -741,8 +742,8 @@ int Solver::div_penalty(const float* vel, const int* act) {
   CB_TRY(divergence(vel, dv, act));
   CB_TRY(dot(dv, n, dv, n, n, S_RW, act));
   for (int a = 0; a < 3; ++a) {
-    const int np = deriv_partials(d, a, 1);
-    CB_TRY(launch_deriv(dv, n, n, nullptr, 0, 0, 1, B, d, a, EPI_SUMSQ, partials, maxparts, act, stream));
+    int np = 0;
+    CB_TRY(launch_deriv(dv, n, n, nullptr, 0, 0, 1, B, d, a, EPI_SUMSQ, partials, maxparts, act, stream, &np));
     CB_TRY(launch_finalize(partials, maxparts, np, slot(S_RW), B, 1.0, true, stream, act));
   }
   note_launches(6);
@@ -815,9 +816,10 @@ int Solver::reg_op(const float* vin, float* out, int op, int epi, const int* act
   CB_TRY(launch_pencil(spec, 3 * nc, B, d, op, dparams, 3, 3, act, stream));
   if (dot_with && fused_dots) {
     const int e2 = (epi == EPI_ADD) ? EPI_ADD_DOT : EPI_STORE_DOT;
+    int np = 0;
     CB_TRY(launch_c2r3d(spec, 3 * nc, out, 3 * n, n, 3, B, d, e2, nullptr, partials, maxparts, act, stream,
-                        dot_with));
-    CB_TRY(launch_finalize(partials, maxparts, c2r_partials(d, 3), slot(dot_slot), B, 1.0, false, stream, act));
+                        dot_with, &np));
+    CB_TRY(launch_finalize(partials, maxparts, np, slot(dot_slot), B, 1.0, false, stream, act));
     note_launches(6);
     return 0;
   }

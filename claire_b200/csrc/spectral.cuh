@@ -53,20 +53,25 @@ int launch_pencil(float2* spec, long long sp, int nprob, const Dims& d, int op,
                   const SpecParams* dparams, int nin, int nout, const int* active, cudaStream_t s,
                   const SpecParams* one = nullptr);
 // Inverse c2r of nf fields with epilogue: out[p*op + f*ofs] = alpha[p]*x (+ out) or sumsq.
+// A reducing epilogue leaves *used partials per problem at partials + p*nparts;
+// the count is that of the variant this launch ran with, so the caller sums what
+// was written whatever becomes of the size's variant in the meantime.  A count
+// above nparts is an error.
 int launch_c2r3d(float2* spec, long long sp, float* out, long long op_, long long ofs, int nf,
                  int nprob, const Dims& d, int epi, const float* alpha, double* partials, int nparts,
-                 const int* active, cudaStream_t s, const float* other = nullptr);
+                 const int* active, cudaStream_t s, const float* other = nullptr, int* used = nullptr);
 
 // Spectral first derivative along one axis (0:x1, 1:x2, 2:x3) of nf real
-// fields with Nyquist set to zero; out = d/dx_axis in (+ out) or sumsq.
+// fields with Nyquist set to zero; out = d/dx_axis in (+ out) or sumsq (partials
+// as in launch_c2r3d).
 int launch_deriv(const float* in, long long ip, long long ifs, float* out, long long op_,
                  long long ofs, int nf, int nprob, const Dims& d, int axis, int epi,
-                 double* partials, int nparts, const int* active, cudaStream_t s);
+                 double* partials, int nparts, const int* active, cudaStream_t s, int* used = nullptr);
 
-// Number of reduction partials a launch with these arguments writes per problem
-// (any_variant: the largest count over the size's FFT variants, for sizing).
-int deriv_partials(const Dims& d, int axis, int nf, bool any_variant = false);
-int c2r_partials(const Dims& d, int nf, bool any_variant = false);
+// Room for the reduction partials of one problem: the largest count over the
+// size's FFT variants.
+int deriv_partials(const Dims& d, int axis, int nf);
+int c2r_partials(const Dims& d, int nf);
 
 // FFT variant of an N-point axis: bit 0 the alternative two-stage radix plan,
 // bit 1 the alternative lines per CTA.  Process-wide, default 0; change it
