@@ -510,11 +510,11 @@ int launch_field_stats(const float* f, long long fp, long long n, int nprob, dou
 }
 
 // Bounded waits on this device that ran out.
-int stage_timeouts(unsigned long long* count, cudaStream_t s) {
+int stage_timeouts(unsigned long long* count) {
   unsigned v = 0;
-  if (cudaMemcpyFromSymbolAsync(&v, g_stage_timeouts, sizeof(unsigned), 0, cudaMemcpyDeviceToHost, s) !=
+  if (cudaMemcpyFromSymbolAsync(&v, g_stage_timeouts, sizeof(unsigned), 0, cudaMemcpyDeviceToHost, nullptr) !=
           cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess)
+      cudaStreamSynchronize(nullptr) != cudaSuccess)
     return (int)cudaGetLastError();
   *count = v;
   return 0;

@@ -209,21 +209,9 @@ long long Solver::estimate_bytes(const claire_b200_opts& o, int B) {
   return bytes;
 }
 
-// A bounded device wait ran out (sl_tile.cuh); report it once, at the next
-// GN-iteration boundary.
-int Solver::check_stage() {
-  unsigned long long t = 0;
-  if (stage_timeouts(&t, stream)) return CB_ERR_CUDA;
-  if (t <= stage_seen) return 0;
-  stage_seen = t;
-  err = "a bounded device wait did not complete within its limit";
-  return CB_ERR_CUDA;
-}
-
 int Solver::init(const claire_b200_opts& o, int Bn) {
   opts = o;
   B = Bn;
-  stage_timeouts(&stage_seen);
   d = Dims{o.nx[0], o.nx[1], o.nx[2]};
   nt = o.nt;
   if (B < 1 || B > 1024 || nt < 1) {
@@ -1836,7 +1824,6 @@ int Solver::step(std::vector<int>& finished, double gttol, int miniter) {
   if (anyacc) CB_TRY(gradient_at_current(acc));
   for (int b = 0; b < B; ++b)
     if (acc[b]) ps[b].iter++;
-  CB_TRY(check_stage());
   if (opts.verbosity > 0) {
     // OptimizationMonitor line (src/TaoInterface.cpp:529-606)
     for (int b = 0; b < B; ++b)
@@ -1867,7 +1854,6 @@ int Solver::finish(const std::vector<int>& sel) {
   CB_TRY(launch_finalize(partials, maxparts, np, slot(S_RR), B, 1.0, false, stream, dact));
   note_launches(2);
   CB_TRY(fetch_scalars());
-  CB_TRY(check_stage());
   const auto t1 = std::chrono::steady_clock::now();
   for (int b = 0; b < B; ++b) {
     if (!sel[b]) continue;

@@ -97,8 +97,6 @@ class Solver {
   cudaStream_t own_stream = nullptr;  // the context's own stream
   std::vector<ProbState> ps;
   std::string err;
-  unsigned long long stage_seen = 0;  // box-copy timeouts of the device already reported
-  int check_stage();                  // CB_ERR_CUDA when a bounded device wait ran out
 
   // device state: one allocation per array, problem p at base + p * stride
   float *mR = nullptr, *mT = nullptr, *v = nullptr, *vtrial = nullptr, *m = nullptr;

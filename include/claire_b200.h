@@ -299,13 +299,12 @@ long long claire_b200_kernel_launches(void);
 
 /* Health of bounded device waits.  A wait on a barrier that runs out is
  * counted in a device word and the kernel returns.
- * claire_b200_stage_timeouts returns the count on the current device (a
- * context's next GN step reports CB_ERR_CUDA when it grew).
+ * claire_b200_stage_timeouts returns the count on the current device.
  * claire_b200_stage_wait_selftest launches one block that waits wait_ns for a
- * copy that is never issued, so the count grows by one and the context stays
- * usable.  The tile gathers themselves stage their boxes with asynchronous
- * copies that each thread waits for as for its own loads: no barrier of theirs
- * can run out.  The reference's interpolation has no device waits
+ * copy that is never issued, so the count grows by one; contexts and servers
+ * are not affected.  The library's other kernels wait on no barrier that could
+ * run out: the tile gathers stage their boxes with asynchronous copies that
+ * each thread waits for as for its own loads.  The reference's interpolation has no device waits
  * (src/interp3.cpp:2492-2719 runs on the host). */
 int claire_b200_stage_timeouts(long long* count);
 int claire_b200_stage_wait_selftest(long long wait_ns, void* stream);

@@ -176,3 +176,21 @@ def test_box_copy_wait_runs_out_cleanly(cb):
     ref = R.interp3(f.astype(np.float64), R.index_grid((n, n, n)) + disp.astype(np.float64))
     assert np.linalg.norm((out - ref).ravel()) <= 1e-5 * np.linalg.norm(ref.ravel())
     assert cb.stage_timeouts() == before + 1  # real copies complete within the limit
+
+
+def test_a_wait_that_ran_out_elsewhere_does_not_fail_a_solve(cb):
+    """The count of waits that ran out is the device's, and no kernel of a solve
+    waits on such a barrier: a self-test between a context's creation and its
+    run leaves the run alone."""
+    import torch
+    mR, mT = c1_32()
+    with cb.CLAIREInterface(opt32(cb)) as ci:
+        ci.set_images(mR, mT)
+        ci.Run()
+        ref = ci.GetSolution()
+    with cb.CLAIREInterface(opt32(cb)) as ci:
+        ci.set_images(mR, mT)
+        cb.stage_wait_selftest(1_000_000)
+        torch.cuda.synchronize()
+        ci.Run()
+        assert np.array_equal(ci.GetSolution(), ref)
