@@ -431,6 +431,7 @@ int launch_interp16(const bf16* f, long long fp, const float* disp, long long dp
   // staged boxes load 4-element chunks as 8-byte words (only when N3 % 4 == 0)
   if (!(d.n3 & 3) && ((reinterpret_cast<uintptr_t>(f) & 7) || (fp & 3))) return (int)cudaErrorInvalidValue;
   if (!tab) {
+    if (nprob != 1 || active) return (int)cudaErrorInvalidValue;  // one field at one map
     int e = allow_smem(k_interp16_direct);
     if (e) return e;
     k_interp16_direct<<<tile_grid(d, 1, 1), kTileThreads, kGatherSmemBytes, s>>>(f, disp, out, d, TileGrid(d));

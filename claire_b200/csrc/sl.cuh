@@ -105,7 +105,7 @@ int launch_interp(const float* f, long long fp, long long ff, const float* disp,
 
 // Same for one bf16 image field per problem (state levels stored in bf16):
 // taps widened to FP32, sums in FP32, the result rounded to bf16.  Without a
-// table: one problem.
+// table: one problem and no mask (anything else is an error).
 int launch_interp16(const bf16* f, long long fp, const float* disp, long long dp, const int4* tab, long long tp,
                     bf16* out, long long op, int nprob, const Dims& d, const int* active, cudaStream_t s);
 
