@@ -797,12 +797,14 @@ int Solver::objective_at(const float* vel, const std::vector<int>& sel) {
 // spectral building blocks
 // ---------------------------------------------------------------------------
 // out = F^-1(symbol F(vin)) with epilogue epi (EPI_SUM: plus addend); with dot_with, out . dot_with
-// (FP64) lands in slot dot_slot (the inverse transform's epilogue sums it).
+// (FP64) lands in slot dot_slot: summed in the inverse transform's epilogue for
+// EPI_STORE and EPI_ADD, in a pass of its own for EPI_SUM, whose epilogue already
+// reads one other array, and where fused_dots is off.
 int Solver::reg_op(const float* vin, float* out, int op, int epi, const int* act, const float* dot_with,
                    int dot_slot, const float* addend) {
   CB_TRY(launch_r2c3d(vin, 3 * n, n, spec, 3 * nc, 3, B, d, act, stream));
   CB_TRY(launch_pencil(spec, 3 * nc, B, d, op, dparams, 3, 3, act, stream));
-  if (dot_with && fused_dots) {
+  if (dot_with && fused_dots && epi != EPI_SUM) {
     const int e2 = (epi == EPI_ADD) ? EPI_ADD_DOT : EPI_STORE_DOT;
     int np = 0;
     CB_TRY(launch_c2r3d(spec, 3 * nc, out, 3 * n, n, 3, B, d, e2, nullptr, partials, maxparts, act, stream,
@@ -811,14 +813,9 @@ int Solver::reg_op(const float* vin, float* out, int op, int epi, const int* act
     note_launches(6);
     return 0;
   }
-  if (dot_with) {
-    CB_TRY(launch_c2r3d(spec, 3 * nc, out, 3 * n, n, 3, B, d, epi, nullptr, nullptr, 0, act, stream));
-    note_launches(5);
-    return dot(out, 3 * n, dot_with, 3 * n, 3 * n, dot_slot, act);
-  }
   CB_TRY(launch_c2r3d(spec, 3 * nc, out, 3 * n, n, 3, B, d, epi, nullptr, nullptr, 0, act, stream, addend));
   note_launches(5);
-  return 0;
+  return dot_with ? dot(out, 3 * n, dot_with, 3 * n, 3 * n, dot_slot, act) : 0;
 }
 
 // out[level j][axis a] = d/dx_a f[level j]
@@ -879,12 +876,8 @@ int Solver::finish_with_reg(const float* vin, float* out, const int* act, const 
     float* bfo = proj ? bf : out;
     CB_TRY(adjoint_sweep(bfo, act));
     if (norec_act) {
-      if (proj) {
-        CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_SUM, norec_act, nullptr, -1, bf));
-        if (dot_with) CB_TRY(dot(out, 3 * n, dot_with, 3 * n, 3 * n, dot_slot, norec_act));
-      } else {
-        CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_ADD, norec_act, dot_with, dot_slot));
-      }
+      if (proj) CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_SUM, norec_act, dot_with, dot_slot, bf));
+      else CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_ADD, norec_act, dot_with, dot_slot));
     }
     if (dot_with) {
       CB_TRY(launch_add_dot(out, bfo, reg_in, dot_with, 3 * n, 3 * n, B, partials, maxparts, rec_act, stream));
@@ -904,9 +897,7 @@ int Solver::finish_with_reg(const float* vin, float* out, const int* act, const 
     return 0;
   }
   CB_TRY(adjoint_sweep(bf, act));
-  CB_TRY(reg_op(vin, out, OP_REG_GRAD, EPI_SUM, act, nullptr, -1, bf));
-  if (dot_with) CB_TRY(dot(out, 3 * n, dot_with, 3 * n, 3 * n, dot_slot, act));
-  return 0;
+  return reg_op(vin, out, OP_REG_GRAD, EPI_SUM, act, dot_with, dot_slot, bf);
 }
 
 // EvaluateGradient at v (src/CLAIRE.cpp:871-1042); the state must be valid for v.

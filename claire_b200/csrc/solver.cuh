@@ -182,9 +182,10 @@ class Solver {
   bool graphs = true, pcg_warm = false;
   // Reg p by recurrence in the PCG where Reg P = c I (CLAIRE_B200_REG_RECURRENCE=0: off)
   bool reg_rec_enabled = true;
-  // p.q and r.z summed inside the inverse transforms' epilogues, which saves
-  // reading both vectors again (8 problems of 128^3: 72.1 -> 71.6 ms, 32 of 64^3:
-  // 41.3 -> 40.7 ms); CLAIRE_B200_FUSED_DOTS=0: separate dot passes
+  // r.z, and p.q where nothing is projected, summed inside the inverse transforms'
+  // epilogues, which saves reading both vectors again (8 problems of 128^3: 72.1 ->
+  // 71.6 ms, 32 of 64^3: 41.3 -> 40.7 ms); CLAIRE_B200_FUSED_DOTS=0: separate dot
+  // passes
   bool fused_dots = true;
   cudaGraphExec_t pcg_exec = nullptr;
   long long pcg_exec_launches = 0;
