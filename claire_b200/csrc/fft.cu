@@ -936,6 +936,13 @@ static int cols_impl(float2* data, long long pstr, long long fstr, int ncols, in
   return (int)cudaGetLastError();
 }
 
+// The fields of a diagonal symbol share a CTA (and the symbol) once that leaves
+// two CTAs per SM; fewer columns run one field per CTA.  One problem of three
+// fields, one field per CTA against shared: 64^3 4.4 and 6.5 us, 192^3 52.3 and
+// 42.7, 256^3 119 and 105; near the line sharing does not pay yet (128 x 150 x 128,
+// 305 CTAs shared: 19.6 and 22.4).
+static bool pencil_shares_fields(int blocks, int nprob) { return (long long)blocks * nprob >= 2 * 148; }
+
 template <int N, int V>
 static int pencil_impl(float2* spec, long long sp, long long fstr, int nprob, const Dims& d, int op,
                        const SpecParams* params, const SpecParams& one, int nin, int nout, const int* active,
@@ -948,10 +955,8 @@ static int pencil_impl(float2* spec, long long sp, long long fstr, int nprob, co
   if (coupled ? (nin != 3 || nout != 3) : nin != nout) return (int)cudaErrorInvalidValue;
   constexpr int T = ColCfg<N, V>::T;
   const bool diag = op == OP_REG_GRAD || op == OP_REG_INV || op == OP_REG_SQRTINV;
-  // the fields of a diagonal symbol share a CTA (and the symbol) once that
-  // leaves two CTAs per SM; fewer columns run one field per CTA
   const int blocks = (ncols + ColCfg<N, V>::C - 1) / ColCfg<N, V>::C;
-  const bool shared = diag && (long long)blocks * nprob >= 2 * 148;
+  const bool shared = diag && pencil_shares_fields(blocks, nprob);
   const dim3 grid(blocks, coupled || shared ? 1 : nin, nprob);
   const size_t sm = col_smem<N, V>(coupled ? 3 : 1, diag);
   int e = 0;
@@ -1153,13 +1158,15 @@ static int spectral3_explicit_impl(const float* in, float* out, float2* spec, co
   const int ncx2 = d.n1 * n3h;
   const dim3 cols((ncx2 + ColCfg<N, V>::C - 1) / ColCfg<N, V>::C, 3, 1);
   const int ncx1 = d.n2 * n3h;
-  const dim3 pen((ncx1 + ColCfg<N, V>::C - 1) / ColCfg<N, V>::C, 1, 1);
+  const int blocks = (ncx1 + ColCfg<N, V>::C - 1) / ColCfg<N, V>::C;
+  const bool shared = pencil_shares_fields(blocks, 1);
+  const dim3 pen(blocks, shared ? 1 : 3, 1);
   k_r2c_rows<N, V><<<rows, RowCfg<N, V>::T, RowCfg<N, V>::smem, s>>>(in, 0, n, spec, 0, nc, nrows, tw, nullptr);
   constexpr int T = ColCfg<N, V>::T;
   const size_t sm = col_smem<N, V>(1);
   k_cols<N, false, V><<<cols, T, sm, s>>>(spec, 0, nc, ncx2, n3h, (long long)d.n2 * n3h, n3h, tw, nullptr);
   k_pencil1<N, V, true><<<pen, T, col_smem<N, V>(1, true), s>>>(
-      spec, 0, nc, 3, d, op, 1.f / (float)((double)d.n1 * d.n2 * d.n3), params, SpecParams{}, tw, nullptr);
+      spec, 0, nc, shared ? 3 : 1, d, op, 1.f / (float)((double)d.n1 * d.n2 * d.n3), params, SpecParams{}, tw, nullptr);
   k_cols<N, true, V><<<cols, T, sm, s>>>(spec, 0, nc, ncx2, n3h, (long long)d.n2 * n3h, n3h, tw, nullptr);
   k_c2r_rows<N, V><<<rows, RowCfg<N, V>::T, RowCfg<N, V>::smem, s>>>(spec, 0, nc, out, 0, n, nrows, tw, EPI_STORE, nullptr,
                                                            nullptr, 0, nullptr, nullptr);
