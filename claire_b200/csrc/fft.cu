@@ -337,32 +337,6 @@ __global__ void __launch_bounds__(ColCfg<N, V>::T, 1024 / ColCfg<N, V>::T)
 // spectral symbols (src/Regularization*.cpp, src/CLAIREStokes.cpp:407-540,
 // src/CLAIREDivReg.cpp:313-460, src/Preprocessing.cpp:1956-2056)
 // ---------------------------------------------------------------------------
-CB_DEVICE float reg_grad_symbol(const SpecParams& q, float kap) {
-  switch (q.norm) {
-    case NORM_L2: return q.beta0;
-    case NORM_H1SN: return q.hd * q.beta0 * kap;
-    case NORM_H1: return q.hd * q.beta0 * (kap + q.beta1);
-    case NORM_H2: return q.beta0 * (kap * kap + q.beta1);
-    case NORM_H2SN: return q.hd * q.beta0 * kap * kap;
-    case NORM_H3: return q.beta0 * (kap * kap * kap + q.beta1);
-    case NORM_H3SN: return q.beta0 * kap * kap * kap;
-    default: return 0.f;
-  }
-}
-
-CB_DEVICE float reg_inv_operator(const SpecParams& q, float kap) {
-  switch (q.norm) {
-    case NORM_L2: return q.beta0;
-    case NORM_H1SN: return kap == 0.f ? q.beta0 : q.beta0 * kap;
-    case NORM_H1: return q.beta0 * (kap + q.beta1);
-    case NORM_H2: return q.beta0 * (kap * kap + q.beta1);
-    case NORM_H2SN: return kap == 0.f ? q.beta0 : q.beta0 * kap * kap;
-    case NORM_H3: return q.beta0 * (kap * kap * kap + q.beta1);
-    case NORM_H3SN: return kap == 0.f ? q.beta0 : q.beta0 * kap * kap * kap;
-    default: return 1.f;
-  }
-}
-
 // Wavenumber data of one spectral column (x2 index i2, x3 index i3) and a
 // spectral element of it along x1 (index i1).
 struct ColumnK {
@@ -378,23 +352,13 @@ CB_DEVICE ColumnK column_k(int i2, int i3, const Dims& d) {
   return c;
 }
 
-// Per-field diagonal operators (one field, component index comp for H3/H3SN).
+// The diagonal operators without a DiagSymbol: the regularisation functional and
+// the Gaussian (one field, component index comp for H3/H3SN).
 CB_DEVICE float2 apply_op1(int op, const SpecParams& q, const Dims& d, int i1, const ColumnK& ck, int comp,
                            float2 x, float s) {
   const float k1 = (float)wavenumber(i1, d.n1);
   const float kap = k1 * k1 + ck.k2 * ck.k2 + ck.k3 * ck.k3;
   switch (op) {
-    case OP_REG_GRAD: {
-      const float sig = s * reg_grad_symbol(q, kap);
-      return make_float2(x.x * sig, x.y * sig);
-    }
-    case OP_REG_INV:
-    case OP_REG_SQRTINV: {
-      float o = reg_inv_operator(q, kap);
-      if (op == OP_REG_SQRTINV) o = sqrtf(o);
-      const float sig = s / o;
-      return make_float2(x.x * sig, x.y * sig);
-    }
     case OP_REG_FUNC: {
       if (q.norm == NORM_L2) {
         const float sig = s * sqrtf(q.beta0);
@@ -459,10 +423,14 @@ CB_DEVICE void apply_op3(int op, const SpecParams& q, const Dims& d, int i1, con
   x[2] = make_float2(g * ck.k3 * kd.x, g * ck.k3 * kd.y);
 }
 
-// The real diagonal operators that run once per Krylov iteration (gradient,
-// inverse and square-root inverse of the regularisation), reduced to
+// The real diagonal operators that run once per Krylov iteration, reduced to
 // sig = s coef (t + b1) or s / (coef (t + b1)) with t a power of kappa, so that
-// one symbol costs a few instructions per element.
+// one symbol costs a few instructions per element:
+//   gradient   L2 beta0, H1SN hd beta0 kappa, H1 hd beta0 (kappa + beta1),
+//              H2SN hd beta0 kappa^2, H2 beta0 (kappa^2 + beta1),
+//              H3SN beta0 kappa^3, H3 beta0 (kappa^3 + beta1)
+//   inverse    1 / the same without hd, the seminorms' symbol beta0 at kappa = 0;
+//              its square root for the square-root inverse
 struct DiagSymbol {
   float s, coef, b1;
   int power;
@@ -475,7 +443,7 @@ struct DiagSymbol {
     power = q.norm == NORM_L2 ? 0 : (h1 ? 1 : (h2 ? 2 : 3));
     const bool semi = q.norm == NORM_H1SN || q.norm == NORM_H2SN || q.norm == NORM_H3SN;
     b1 = (semi || q.norm == NORM_L2) ? 0.f : q.beta1;
-    // the hd factor of the gradient symbols (reg_grad_symbol's table)
+    // the norms whose gradient symbol has the factor hd
     const bool hd = q.norm == NORM_H1SN || q.norm == NORM_H1 || q.norm == NORM_H2SN;
     coef = (!inv && hd) ? q.hd * q.beta0 : q.beta0;
     keep0 = inv && semi;

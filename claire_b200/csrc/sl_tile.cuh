@@ -93,9 +93,6 @@ CB_DEVICE unsigned tile_div(unsigned t, unsigned nb, unsigned m) {
   return q * nb > t ? q - 1 : q;
 }
 
-// x1 plane of a thread's point a, from its first.
-CB_DEVICE constexpr int plane_of(int a) { return a; }
-
 // This thread's points in the CTA's tile: 4 consecutive x1 planes of one row
 // and column.  Coordinates are clamped to the grid: a point beyond it repeats
 // the last one inside (same tile, so the same box), which makes every load and
@@ -107,7 +104,7 @@ struct TileThread {
   unsigned vmask;   // bit a: point a lies inside the grid
   unsigned idx0, plane;
   CB_DEVICE bool valid(int a) const { return (vmask >> a) & 1u; }
-  CB_DEVICE int step(int a) const { return min(plane_of(a), amax); }
+  CB_DEVICE int step(int a) const { return min(a, amax); }
   CB_DEVICE int x1(int a) const { return x1_ + step(a); }
   CB_DEVICE unsigned idx(int a) const { return idx0 + (unsigned)step(a) * plane; }
 };
@@ -602,7 +599,7 @@ CB_DEVICE void gather_tile(unsigned sb, const PointList& list, const Src& src, c
     const int id = list.id[i];
     int l1, l2, l3;
     tile_local(id / kTilePts, l1, l2, l3);
-    const int x1 = t1 + l1 + plane_of(id % kTilePts), x2 = t2 + l2, x3 = t3 + l3;
+    const int x1 = t1 + l1 + id % kTilePts, x2 = t2 + l2, x3 = t3 + l3;
     const unsigned at = (unsigned)x1 * tt.plane + (unsigned)x2 * (unsigned)d.n3 + (unsigned)x3;
     float de[3], s[3], w1[4], w2[4], w3[4];
     src.at(de, at, d);
