@@ -56,8 +56,8 @@ static const float2* twiddles(int n) {
 
 // Lengths with a plan on every axis, and the extra lengths the column and
 // pencil passes (axes x1, x2) also take: 150 = 10 x 15 (the x2 length of the
-// reference's example brains, 128 x 150 x 128).  Row passes need N % 16 == 0
-// (16-byte row loads, whole float4 per thread).
+// reference's example brains, 128 x 150 x 128).  Row passes have no plan for it:
+// their R0 is a power of two (RowPlan).
 bool fft_size_supported(int n) {
   switch (n) {
     case 16: case 32: case 48: case 64: case 96: case 128: case 192: case 256: return true;
@@ -85,10 +85,15 @@ constexpr int row_pairs(int r1, int v) {
 // Row kernels (bound by global traffic: three 256^3 fields 68 us r2c and 70 us
 // c2r against a floor of 62; 150 and 165 us when rows were transposed through
 // padded shared memory on the way in and out; 128^3: 12.4 and 11.4 against 20
-// and 21): a warp's lanes are neighbouring butterflies of a few lines, so
-// the shared layout y[line, k0, j] at line * PL + k0 * PK + j is read and
-// written without bank conflicts: A (lanes over j, then lines) needs
-// PL = R1 (mod 16 float2), B (lanes over k0) an odd PK.
+// and 21): a warp's lanes are neighbouring butterflies of a few lines.  The
+// shared layout is y[line, k0, j] at line * PL + k0 * PK + j; 64-bit accesses are
+// served by half-warps.  A (lanes over j, then lines) has no bank conflicts, as
+// PL = R1 (mod 16 float2); B (lanes over k0, odd PK) has none with R0 = 16 and at
+// 4 x 4, 4 x 12 and 8 x 8, and two-way ones in the other plans with R0 < 16, where
+// the lines of a half-warp meet.  The twiddles tw[j k0] take 1.1 to 2.2
+// wavefronts a half-warp on average, 8 at worst (R0 = 16, j a multiple of 8).
+// Counted at 128^3 (16 x 8): 25% of r2c's shared wavefronts, 18% of c2r's and 22%
+// of the derivative's are conflicts, all of them twiddles.
 template <int N, int V> struct RowCfg {
   static constexpr int R0 = RowPlan<N, V>::R0, R1 = RowPlan<N, V>::R1;
   static constexpr int P = row_pairs(R1, V), T = P * R1;
@@ -104,8 +109,9 @@ template <int N, int V> struct RowCfg {
 // adjacent columns in both butterflies, so
 // every global access is a run of C float2 and every shared access a run of
 // 16 consecutive float2 per half-warp (64-bit accesses are served by half-warps):
-// no bank conflicts at pitch C.  The CTA has one thread per A butterfly
-// (C * R1), 256 at most.
+// no bank conflicts by the layout at pitch C (counted at 128^3: 6% of the
+// wavefronts, 11% with the pencil's symbols).  The CTA has one thread per A
+// butterfly (C * R1), 256 at most.
 template <int N, int V = 0> struct ColCfg {
   static constexpr int C = (V & 2) ? ColLines<N>::alt : ColLines<N>::base;
   static constexpr int R0 = Plan<N, V>::R0, R1 = Plan<N, V>::R1;
@@ -948,6 +954,8 @@ static bool axes_supported(const Dims& d) {
 }
 static bool cubic_supported(const Dims& d) { return d.n1 == d.n2 && d.n2 == d.n3 && axes_supported(d); }
 
+// Inputs of the row passes have to start on 16 bytes, which callers rely on being
+// told (the kernels load single floats and would take any).
 int launch_r2c3d(const float* in, long long ip, long long ifs, float2* spec, long long sp, int nf,
                  int nprob, const Dims& d, const int* active, cudaStream_t s) {
   if (!axes_supported(d) || !aligned16(in) || ((ip | ifs) & 3)) return (int)cudaErrorInvalidValue;

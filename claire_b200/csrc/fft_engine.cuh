@@ -217,7 +217,12 @@ template <int R, bool INV> struct Dft {
 // factorization (the other factor order, or 16 x 4 for 64); the autotuner
 // picks per grid size whichever runs faster (Plan0 where there is none).  32
 // points: 8 x 4 columns and 4 x 8 rows run the tuner's work in 35.5 us on 8
-// problems, the other order in 39.1 (34.5 both on one).
+// problems, the other order in 39.1 (34.5 both on one).  Speed is not the only
+// reason: the order of the stages decides how roundoff falls, and with it the
+// outcome of solves at 32^3 that sit on it (the two-level preconditioner's
+// mismatch against the oracle's, Gauss-Newton counts of H3 solves whose inverse
+// symbol is 1e8 at k = 0).  Of the four combinations of column and row orders,
+// together with the gathers' order of sums, the tests of those pass with this one.
 template <int N> struct Plan0;
 template <> struct Plan0<16> { static constexpr int R0 = 4, R1 = 4; };
 template <> struct Plan0<32> { static constexpr int R0 = 8, R1 = 4; };

@@ -105,7 +105,7 @@ extern "C" int claire_b200_reg_apply_noalloc(const float* v, float* out, const i
       kind < CB_REG_GRADIENT || kind > CB_REG_SQRTINVERSE)
     return CB_ERR_ARG;
   if (nx[0] <= 0 || nx[1] <= 0 || nx[2] <= 0) return CB_ERR_ARG;
-  // the transform kernels read and write 16-byte vectors
+  // part of this entry point's contract
   if ((reinterpret_cast<uintptr_t>(v) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return CB_ERR_ARG;
   if (!(nx[0] == nx[1] && nx[1] == nx[2])) return CB_ERR_UNSUPPORTED;
   if (nx[0] > kMaxN) return CB_ERR_TOO_LARGE;

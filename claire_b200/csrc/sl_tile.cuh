@@ -11,9 +11,12 @@
 // shared memory; tiles whose box is too large (large, rough displacements)
 // gather from global memory instead.
 //
-// What bounds a gather is the shared-memory data path (64 words a point, and
-// bank conflicts on top where floors change inside a warp) and, close behind,
-// instruction issue.  The two points of a pair nearly always have the same
+// What bounds a gather is the SM's data path and, close behind, instruction
+// issue.  Counted per 32 points of one field at 128^3 (adjoint step, half the
+// benchmark's velocity): 91 wavefronts, of which 50 taps and box copies, 22 bank
+// conflicts where floors change inside a warp, 16 global loads and stores and 3
+// spilled registers (64 a thread); three fields at one map 99 a field with 5 of
+// spills, the three components of a characteristic 96 with 10.  The two points of a pair nearly always have the same
 // floor(d) (all but 3-10% of them on the benchmark's velocities): their stencils
 // then share 3 of 5 planes, and one pass over 5 planes of 16 words serves both
 // (40 words a point).  A pair whose floors differ gathers its first point in
@@ -145,7 +148,13 @@ CB_DEVICE TileThread tile_thread(const Dims& d, const TileGrid& tg) {
 
 // x3 row pitches of a staged box: 48 floats (16 mod 32 banks), or 32 where only
 // that fits (strong maps; the two rows of a warp then share their banks, which
-// is far cheaper than gathering from global memory)
+// is far cheaper than gathering from global memory).  192 x 192 x 256, one field,
+// every box of the map alike, against pitches 32 / 64 with a plane offset that
+// keeps the two rows apart and 32 KB a box: 169 rows of 20 floats 125 us (140), 225
+// rows (pitch 32) 174 (155), 256 and 289 rows 176 (261, global memory), 324 rows
+// (global memory) 268 (262).  Rows of 49 to 64 floats go to global memory, 257-301
+// us, which pitch 64 served in 178: such a map stretches x3 by 2.7 and more over a
+// whole tile, and code for a third pitch cost every gather of three fields 1 to 3%.
 constexpr int kPitch = 48, kPitchTight = 32;
 
 struct TileBox {
@@ -472,7 +481,9 @@ CB_DEVICE f32x2 row_sums(const f32x2 (&x)[NC], const f32x2 (&w3)[NC]) {
 
 // Weights of points A and B (fractions s, t): along x1, along x2 as row pairs
 // (r, r + 2), so that a sum runs over neighbouring rows before the two halves
-// meet, along x3 duplicated.
+// meet, along x3 duplicated.  The choice against pairs (r, r + 1) is one
+// of roundoff: solves that sit on it (H3 with beta 1e-4 at 32^3) keep the oracle's
+// Gauss-Newton counts with this order of sums and not with the other.
 struct PairWeights {
   float w1[2][4];
   f32x2 w2[2][2], w3[2][4];
