@@ -425,9 +425,9 @@ def tune(cb, sizes, nbatch):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_gather_scale launch over
-# one 128^3 problem of the workload (42,297,344 bytes; ncu, the command in
+# one 128^3 problem of the workload (42,398,208 bytes; ncu, the command in
 # profiles/k_gather_scale_128.md), per point
-GATHER_SCALE_DRAM_BYTES_PER_POINT = 42297344 / 128 ** 3
+GATHER_SCALE_DRAM_BYTES_PER_POINT = 42398208 / 128 ** 3
 # l1tex__data_pipe_lsu_wavefronts_mem_shared.sum of the same capture (2.99 M
 # shared-memory wavefronts for 128^3 points: the words two points of a pair
 # read together, and the 16-byte copies of the boxes), per point; a B200 SM
